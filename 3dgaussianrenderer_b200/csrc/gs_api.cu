@@ -539,7 +539,7 @@ int run_frame_onesweep(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams
     ra.tile_counter = &dc->raster_tile;
     ra.rec_chunk = cfg.raster_chunk;
     ra.rec_persistent = cfg.raster_persistent;
-    launch_raster(ra, cfg.tile_w, cfg.tile_h, cfg.termination, num_views > 1, ctx->num_sms, st);
+    launch_raster(ra, cfg.tile_w, cfg.tile_h, cfg.termination, ctx->num_sms, st);
     GS_CUDA(cudaGetLastError());
     GS_CUDA(cudaEventRecord(ctx->ev[5], st));
     GS_CUDA(cudaMemcpyAsync(&ctx->h_counters->err, &dc->err, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -775,11 +775,11 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
             rg.num_tiles_total = t1 - t0;
             // a persistent group launch starts its own queue from zero
             if (rg.rec_persistent) GS_CUDA(cudaMemsetAsync(&dc->raster_tile, 0, sizeof(unsigned long long), st));
-            launch_raster(rg, cfg.tile_w, cfg.tile_h, cfg.termination, false, ctx->num_sms, st);
+            launch_raster(rg, cfg.tile_w, cfg.tile_h, cfg.termination, ctx->num_sms, st);
             GS_CUDA(record(ctx->ev_group[g], st, capturing));
         }
     } else {
-        launch_raster(ra, cfg.tile_w, cfg.tile_h, cfg.termination, p.num_views > 1, ctx->num_sms, st);
+        launch_raster(ra, cfg.tile_w, cfg.tile_h, cfg.termination, ctx->num_sms, st);
     }
     GS_CUDA(cudaGetLastError());
     GS_CUDA(record(ctx->ev[5], st, capturing));
@@ -1768,7 +1768,7 @@ int gs_stage_raster(const gs_camera* cam, const gs_render_cfg* cfg, const int32_
     ra.conic = (const float4*)d_conic;
     ra.color = (const float4*)d_color;
     ra.t_min = cfg->t_min;
-    launch_raster(ra, cfg->tile_w, cfg->tile_h, cfg->termination, false, device_sm_count(), (cudaStream_t)stream);
+    launch_raster(ra, cfg->tile_w, cfg->tile_h, cfg->termination, device_sm_count(), (cudaStream_t)stream);
     GS_CUDA(cudaGetLastError());
     return GS_OK;
 }

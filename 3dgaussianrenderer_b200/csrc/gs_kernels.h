@@ -240,8 +240,8 @@ struct SortScratch {
 };
 
 struct RasterArgs {
-    ViewParams view0;                 // single-view kernel: the view, by value
-    const ViewParams* views;          // persistent kernel: all views
+    ViewParams view0;                 // the first view, by value (the only one of a single-view launch)
+    const ViewParams* views;          // all views
     int32_t num_views;
     int32_t write_empty;              // 1: tiles without entries are written as (0,0,0,0)
     int64_t num_tiles_total;          // sum of the views' tiles (of this launch's tiles when tile_base is used)
@@ -253,7 +253,7 @@ struct RasterArgs {
     const float4* color;
     const float4* rec;                // 3 float4 per value (record kernel); null: use xy/conic/color
     float t_min;
-    unsigned long long* tile_counter; // persistent variant only
+    unsigned long long* tile_counter; // persistent record raster only
     // tile-bucket frames: a tile of at most fused_cap keys is sorted by its
     // raster CTA from the bucketed (depth << 32 | slot) keys; `values` then
     // only holds the order of the larger tiles.  keys == null: `values`
@@ -304,8 +304,7 @@ int sort_passes(int key_bits);
 
 void launch_ranges(const uint64_t* keys, int64_t num_items, const int64_t* d_num_items, int32_t* ranges,
                    cudaStream_t st);
-void launch_raster(const RasterArgs& a, int tile_w, int tile_h, int termination, bool persistent, int num_sms,
-                   cudaStream_t st);
+void launch_raster(const RasterArgs& a, int tile_w, int tile_h, int termination, int num_sms, cudaStream_t st);
 
 // Scene storage order (gs_scene.cu): 30-bit Morton codes of the centres over
 // the box [lo, hi] with values = index, then the gather of every scene array
