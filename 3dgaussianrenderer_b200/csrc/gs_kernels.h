@@ -187,8 +187,8 @@ constexpr int kTileSortSmemKeys = 4096;
 // 1024-thread CTA (tile_sort_huge_kernel); larger ones by passes through
 // global memory.
 constexpr int kTileSortHugeKeys = 16384;
-// Keys a tile may have to be sorted inside its raster CTA (TW * TH / 2
-// threads, 8 keys each); larger tiles are sorted ahead of the raster.
+// Keys a tile may have to be sorted inside its raster CTA (8 per two
+// pixels); larger tiles are sorted ahead of the raster.
 constexpr int kFusedIpt = 8;
 inline int fused_tile_capacity(int tile_w, int tile_h) { return tile_w * tile_h / 2 * kFusedIpt; }
 constexpr int kTileScanItems = 1024;  // tiles per scan block
@@ -262,8 +262,8 @@ struct RasterArgs {
     const int32_t* slot_gi;
     int32_t fused_cap;
     const int32_t* order;             // non-null: CTA (or queue entry) k rasterises tile order[k]
-    // record raster (GS_TERM_TMIN) knobs: entries culled and staged per warp
-    // step (32 or 64), and a persistent grid over the atomic tile queue
+    // record raster (GS_TERM_TMIN) knobs: entries between two tests of whether
+    // a block is done (32 or 64), and a persistent grid over the atomic tile queue
     // (tile_counter, zero at launch) instead of one CTA per tile
     int32_t rec_chunk;
     int32_t rec_persistent;

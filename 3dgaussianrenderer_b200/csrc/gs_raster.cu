@@ -178,38 +178,20 @@ __device__ __forceinline__ void store_pixel(const ViewParams& v, const int px, c
 // reads the slots from there.  Larger tiles were sorted ahead of the raster
 // and are read from `values`.
 
-// NT threads sort up to CAP keys (CAP / NT keys per thread).
-template <int NT, int CAP = NT * kFusedIpt>
-struct FusedSortSmem {
-    uint64_t k[CAP];
-    int32_t v[CAP];
-    int32_t bexcl[256];
-    int32_t dcount[256];
-    int32_t scan[NT / 32];
-    uint64_t red[2 * (NT / 32)];
-};
-
-// Returns the tile's sorted keys in shared memory, or null when the order
-// is in a.values.  Every thread of the CTA must call it.
+// Sorts a tile of up to CAP keys with the CTA's NT threads (CAP / NT keys
+// per thread).  Returns the tile's sorted keys (sm.k), or null when the order
+// is in a.values.  Every thread of the CTA must call it; where it sorts, it
+// ends with a barrier.
 template <int NT, int CAP>
 __device__ __forceinline__ const uint64_t* fused_sort(const RasterArgs& a, const int first, const int count,
-                                                      FusedSortSmem<NT, CAP>& fs)
+                                                      const tilesort::Smem& sm)
 {
     if (!a.keys || count > a.fused_cap) return nullptr;
     if (count == 1) {
-        if (threadIdx.x == 0) fs.k[0] = a.keys[first];
+        if (threadIdx.x == 0) sm.k[0] = a.keys[first];
         __syncthreads();
-        return fs.k;
+        return sm.k;
     }
-    tilesort::Smem sm;
-    sm.k = fs.k;
-    sm.v = fs.v;
-    sm.whist = reinterpret_cast<uint32_t*>(fs.k);
-    sm.bexcl = fs.bexcl;
-    sm.dcount = fs.dcount;
-    sm.scan = fs.scan;
-    sm.red = fs.red;
-    sm.run = nullptr;
     const uint64_t* src = a.keys + first;
     if (count <= NT)
         tilesort::sort_tile<NT, 1>(src, count, a.slot_gi, sm, a.sort_prefix_bits);
@@ -221,7 +203,7 @@ __device__ __forceinline__ const uint64_t* fused_sort(const RasterArgs& a, const
         tilesort::sort_tile<NT, 8>(src, count, a.slot_gi, sm, a.sort_prefix_bits);
     else
         tilesort::sort_tile<NT, CAP / NT>(src, count, a.slot_gi, sm, a.sort_prefix_bits);
-    return fs.k;
+    return sm.k;
 }
 
 // Slot of the idx-th entry of the tile whose list starts at `first`.
@@ -340,7 +322,7 @@ __device__ __forceinline__ bool wild_entry(const RefSmem& sm, const int j)
 template <int TW, int TH>
 __device__ __forceinline__ void raster_ref_tile(const RasterArgs& a, const ViewParams& v, const int64_t gtile,
                                                 const int local_tile, RefSmem& sm,
-                                                FusedSortSmem<RefShape<TW, TH>::NT, RefShape<TW, TH>::CAP>& fs)
+                                                const tilesort::Smem& ts)
 {
     using S = RefShape<TW, TH>;
     constexpr int NC = S::NC;
@@ -364,7 +346,7 @@ __device__ __forceinline__ void raster_ref_tile(const RasterArgs& a, const ViewP
         }
         return;
     }
-    const uint64_t* sk = fused_sort(a, first, count, fs);
+    const uint64_t* sk = fused_sort<S::NT, S::CAP>(a, first, count, ts);
     // pixel corner sample, gaussian_render.cu:701-704
     const f2 cy = f2_pack((float)py0 * v.texel_y - 1.0f, (float)py1 * v.texel_y - 1.0f);
     float cx[NC];
@@ -438,10 +420,22 @@ __global__ void __launch_bounds__(RefShape<TW, TH>::NT, 640 / RefShape<TW, TH>::
 {
     using S = RefShape<TW, TH>;
     __shared__ RefSmem sm;
-    __shared__ FusedSortSmem<S::NT, S::CAP> fs;
+    __shared__ uint64_t s_k[S::CAP];
+    __shared__ int32_t s_v[S::CAP];
+    __shared__ int32_t s_bexcl[256], s_dcount[256], s_scan[S::NT / 32];
+    __shared__ uint64_t s_red[2 * (S::NT / 32)];
+    tilesort::Smem ts;
+    ts.k = s_k;
+    ts.v = s_v;
+    ts.whist = reinterpret_cast<uint32_t*>(s_k);
+    ts.bexcl = s_bexcl;
+    ts.dcount = s_dcount;
+    ts.scan = s_scan;
+    ts.red = s_red;
+    ts.run = nullptr;
     const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[blockIdx.x]) : (int64_t)blockIdx.x + a.view0.tile_offset;
     const ViewParams& v = view_of_tile(a, gtile);
-    raster_ref_tile<TW, TH>(a, v, gtile, (int)(gtile - v.tile_offset), sm, fs);
+    raster_ref_tile<TW, TH>(a, v, gtile, (int)(gtile - v.tile_offset), sm, ts);
 }
 
 template <int TW, int TH>
@@ -458,169 +452,258 @@ __global__ void __launch_bounds__(TW * TH, 2048 / (TW * TH) * 5 / 8) raster_kern
 // ---- GS_TERM_TMIN from raster records --------------------------------------
 //
 // The frame pipeline's kernel for the T_min mode.  One CTA per tile (all
-// views' tiles in one grid), no CTA-wide barrier: each warp owns an 8x8
-// pixel block, two pixels per lane (rows y and y + 4, same column), and
-// walks the tile's sorted list on its own, 32 entries at a time -- lane l
-// loads entry l's record (48 bytes, gathered through L1, shared by the
-// tile's warps) and tests its cull extents against the block; the
-// survivors are packed in list order into per-warp shared-memory slots
-// (rank = popcount of the ballot below the lane) and every lane blends them
-// into both its pixels.  Every lane reads every survivor, so the slots hold
-// each value once (36 bytes: x, A, B, L, y, C and the colour): the
-// shared-memory reads, not the arithmetic, bound this loop, and duplicated
-// pair operands would double them.  The column terms of the exponent
-// (A dx^2 + L, B dx) are formed once per lane and shared by its two pixels;
-// the weights and T are updated as one packed f32x2 pair.
+// views' tiles in one grid), no CTA-wide barrier after the tile's sort: each
+// warp owns BPW 8x8 pixel blocks side by side (2, or 1 where a tile is one
+// block), 32 / BPW lanes to a block, and walks the tile's sorted list on its
+// own, 32 entries at a time -- a lane tests the cull extents of one entry's
+// record (48 bytes, gathered through L1, shared by the tile's warps) against
+// the blocks; each block's survivors are copied in list order into its own
+// shared-memory slots (rank = popcount of the ballot below the lane) and the
+// block's lanes blend them into their pixels, BPW columns x 2 rows each.  The
+// two halves of a warp walk their blocks' slots side by side; the shorter
+// list is filled up with entries of weight zero (7 % more evaluations on a
+// 1080p view of 1M Gaussians).
 // Blend per pixel: alpha = 2^(A dx^2 + B dx dy + C dy^2 + L) (opacity
 // folded in as L = log2(opacity); the conics are positive definite, so
-// alpha <= opacity), w = T alpha, colour += rgb w, T -= w.  A warp stops
-// after the chunk in which all its pixels reached T < t_min; a pixel that
-// got there earlier keeps blending until then, which adds less than t_min
-// to its colour (the w that follow sum to less than its T).
+// alpha <= opacity), w = T alpha, colour += rgb w, T -= w, in packed f32x2
+// pairs of a column's two rows.  A block stops after the chunk in which all
+// its pixels reached T < t_min; a pixel that got there earlier keeps blending
+// until then, which adds less than t_min to its colour (the w that follow sum
+// to less than its T).
+//
+// Every lane of a block reads every survivor of it.  With one block per warp
+// and two pixels per lane those reads took 9 cycles of the SM's shared-memory
+// path per 64 evaluations and bound the loop; two blocks per warp, four
+// pixels per lane, halve them, share the row term (dy) and the column terms
+// (A dx^2 + L, B dx) among the pixels and leave the FP32 pipe (38 cycles per
+// entry of a warp, 63 % busy) and the ex2 unit (32 cycles, 53 %) as the bound.
+// Raster of the 64-view batch of 3M Gaussians 14.7 -> 12.8 ms, of eight
+// 1280x720 views of 1M 0.99 -> 0.83 ms, of one 1080p view 0.195 -> 0.175 ms.
+// 640 threads per SM (96 registers): 768 with 80 registers spill in the sort
+// and take 13.2 ms, 896 and 1024 take 14.0 ms.
+template <int TW, int TH>
+struct RecShape {
+    static constexpr int BPW = TW / 8;              // 8x8 blocks per warp
+    static constexpr int NT = TW * TH / (2 * BPW);  // threads: 2 BPW pixels each
+    static constexpr int CAP = TW * TH / 2 * kFusedIpt;
+};
 
-// Shared memory of the record raster: per-warp survivor slots (CHUNK per
-// warp) and the fused tile sort.
-template <int TW, int TH, int CHUNK>
-struct RecSmem {
-    static constexpr int NW = TW * TH / 64;
-    float4 s[NW][CHUNK];  // (x, A, B, L)
-    float4 q[NW][CHUNK];  // (y, C, red, green)
-    float b[NW][CHUNK];   // blue
-    FusedSortSmem<TW * TH / 2> fs;
+// Shared memory of the record raster: the sort's buffers and, once the tile
+// is sorted, in their place the tile's slots in blend order and every block's
+// survivors, double-buffered.
+constexpr int kRecStep = 32;  // entries a warp culls and stages at a time
+template <int TW, int TH>
+union RecSmem {
+    using S = RecShape<TW, TH>;
+    static constexpr int NB = TW * TH / 64;
+    struct {
+        uint64_t k[S::CAP];
+        int32_t v[S::CAP];
+        int32_t bexcl[256];
+        int32_t dcount[256];
+        int32_t scan[S::NT / 32];
+        uint64_t red[2 * (S::NT / 32)];
+    } sort;
+    struct {
+        uint32_t order[S::CAP];
+        float4 con[NB][2][kRecStep];  // (A, B, C, L)
+        float4 col[NB][2][kRecStep];  // (red, green, blue, -)
+        float2 xy[NB][2][kRecStep];
+    } r;
 };
 
 // One tile of the record raster.  Every thread of the CTA must call it (the
-// fused sort synchronises the CTA).  CHUNK = the entries a warp culls and
-// stages in shared memory per step, the raster's batch of Gaussians (32 or
-// 64: R = CHUNK / 32 records per lane).
+// fused sort synchronises the CTA).  CHUNK (32 or 64) = the entries between
+// two tests of whether a block is done.
 template <int TW, int TH, int CHUNK>
-__device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64_t gtile, RecSmem<TW, TH, CHUNK>& sm)
+__device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64_t gtile, RecSmem<TW, TH>& sm)
 {
-    constexpr int WX = TW / 8;
-    constexpr int R = CHUNK / 32;
+    using S = RecShape<TW, TH>;
+    constexpr int BPW = S::BPW;
+    constexpr int LPB = 32 / BPW;  // lanes per block
+    constexpr int LX = 8 / BPW;    // lanes across a block
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const ViewParams& v = view_of_tile(a, gtile);
     const int local_tile = (int)(gtile - v.tile_offset);
     const int first = __ldg(&a.ranges[2 * gtile]);
-    const int last = __ldg(&a.ranges[2 * gtile + 1]);
+    const int count = __ldg(&a.ranges[2 * gtile + 1]) - first;
     const int tx = local_tile % v.tiles_x, ty = local_tile / v.tiles_x;
-    const int wx0 = tx * TW + (warp % WX) * 8, wy0 = ty * TH + (warp / WX) * 8;
-    const int px = wx0 + (lane & 7), py0 = wy0 + (lane >> 3), py1 = py0 + 4;
-    const bool in0 = px < v.width && py0 < v.height;
-    const bool in1 = px < v.width && py1 < v.height;
-    if (last - first <= 0) {
+    const int wx0 = tx * TW, wy0 = ty * TH + warp * 8;  // the warp's blocks: (wx0 + 8 b, wy0)
+    const int half = lane / LPB, sub = lane % LPB;
+    const int px = wx0 + 8 * half + (sub % LX) * BPW, py0 = wy0 + sub / LX, py1 = py0 + 4;
+    const bool iny0 = py0 < v.height, iny1 = py1 < v.height;
+    if (count <= 0) {
         if (a.write_empty) {
-            if (in0) v.out[(int64_t)py0 * v.width + px] = make_uchar4(0, 0, 0, 0);
-            if (in1) v.out[(int64_t)py1 * v.width + px] = make_uchar4(0, 0, 0, 0);
+#pragma unroll
+            for (int c = 0; c < BPW; ++c) {
+                if (px + c >= v.width) continue;
+                if (iny0) v.out[(int64_t)py0 * v.width + px + c] = make_uchar4(0, 0, 0, 0);
+                if (iny1) v.out[(int64_t)py1 * v.width + px + c] = make_uchar4(0, 0, 0, 0);
+            }
         }
         return;
     }
-    const uint64_t* sk = fused_sort<TW * TH / 2>(a, first, last - first, sm.fs);
-    const float cx = (float)px * v.texel_x - 1.0f;
-    const float cy0 = (float)py0 * v.texel_y - 1.0f;
-    const float cy1 = (float)py1 * v.texel_y - 1.0f;
-    const float bx0 = (float)wx0 * v.texel_x - 1.0f, bx1 = (float)(wx0 + 7) * v.texel_x - 1.0f;
+    const bool sorted_here = a.keys && count <= a.fused_cap;
+    if (sorted_here) {
+        tilesort::Smem ts;
+        ts.k = sm.sort.k;
+        ts.v = sm.sort.v;
+        ts.whist = reinterpret_cast<uint32_t*>(sm.sort.k);
+        ts.bexcl = sm.sort.bexcl;
+        ts.dcount = sm.sort.dcount;
+        ts.scan = sm.sort.scan;
+        ts.red = sm.sort.red;
+        ts.run = nullptr;
+        fused_sort<S::NT, S::CAP>(a, first, count, ts);
+        // the keys give way to their slots
+        uint32_t o[S::CAP / S::NT];
+#pragma unroll
+        for (int i = 0; i < S::CAP / S::NT; ++i) {
+            const int p = i * S::NT + (int)threadIdx.x;
+            if (p < count) o[i] = (uint32_t)sm.sort.k[p];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < S::CAP / S::NT; ++i) {
+            const int p = i * S::NT + (int)threadIdx.x;
+            if (p < count) sm.r.order[p] = o[i];
+        }
+        __syncthreads();
+    }
+    auto slot = [&](const int j) {
+        return sorted_here ? (int)sm.r.order[j] : __ldg(&a.values[first + j]);
+    };
+    const f2 cy = f2_pack((float)py0 * v.texel_y - 1.0f, (float)py1 * v.texel_y - 1.0f);
     const float by0 = (float)wy0 * v.texel_y - 1.0f, by1 = (float)(wy0 + 7) * v.texel_y - 1.0f;
-    // pixels outside the image start done (T = 0)
-    f2 TT = f2_pack(in0 ? 1.0f : 0.0f, in1 ? 1.0f : 0.0f);
-    float R0 = 0.0f, R1 = 0.0f, G0 = 0.0f, G1 = 0.0f, B0 = 0.0f, B1 = 0.0f;
+    float cx[BPW], bx0[BPW], bx1[BPW];
+    f2 T[BPW], CR[BPW], CG[BPW], CB[BPW];
+    bool out = true;
+#pragma unroll
+    for (int c = 0; c < BPW; ++c) {
+        cx[c] = (float)(px + c) * v.texel_x - 1.0f;
+        bx0[c] = (float)(wx0 + 8 * c) * v.texel_x - 1.0f;
+        bx1[c] = (float)(wx0 + 8 * c + 7) * v.texel_x - 1.0f;
+        // pixels outside the image start done (T = 0)
+        const bool in0 = px + c < v.width && iny0, in1 = px + c < v.width && iny1;
+        T[c] = f2_pack(in0 ? 1.0f : 0.0f, in1 ? 1.0f : 0.0f);
+        CR[c] = CG[c] = CB[c] = f2_dup(0.0f);
+        out = out && !in0 && !in1;
+    }
     const float tmin = a.t_min;
     const unsigned lt = lanemask_lt();
-    bool done = !in0 && !in1;
+    // block b is done when all its lanes are: bits [LPB b, LPB b + LPB)
+    unsigned donemask = __ballot_sync(kFull, out);
+    auto block_done = [&](const int b) {
+        const unsigned m = BPW == 1 ? kFull : 0xFFFFu << (16 * b);
+        return (donemask & m) == m;
+    };
+    const int blk = BPW * warp + half;  // this lane's block in the tile
 
-    // each chunk's cull records are loaded one chunk ahead, so their
-    // latency overlaps the blend of the chunk before
-    float4 qn[R];
-    const float4* rpn[R];
+    // Software pipeline over steps of 32 entries: while step i is blended, the
+    // survivors of step i + 1 are on their way into the other buffer (cp.async),
+    // the cull records of step i + 2 into registers and the slots of step
+    // i + 3 are read.
+    auto load_slot = [&](const int j) { return j < count ? slot(j) : -1; };
+    auto load_cull = [&](const int s) { return s >= 0 ? __ldg(a.rec + 3 * (int64_t)s) : make_float4(0.f, 0.f, 0.f, 0.f); };
+    int cnt[BPW];  // survivors of the step staged last
+    auto stage = [&](const int s, const float4 q, const int buf) {
+        const bool row = s >= 0 && (q.y - q.w <= by1) && (q.y + q.w >= by0);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        qn[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-        rpn[r] = nullptr;
-        if (first + 32 * r + lane < last) {
-            rpn[r] = a.rec + 3 * (int64_t)slot_at(a, sk, first, 32 * r + lane);
-            qn[r] = __ldg(rpn[r]);
-        }
-    }
-    for (int base = first; base < last; base += CHUNK) {
-        if (__all_sync(kFull, done)) break;
-        bool keep[R];
-        unsigned bal[R];
-        const float4* rp[R];
-        float4 q0[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int j = base + 32 * r + lane;
-            q0[r] = qn[r];  // (x, y, ext_x, ext_y)
-            rp[r] = rpn[r];
-            keep[r] = j < last && (q0[r].x - q0[r].z <= bx1) && (q0[r].x + q0[r].z >= bx0) &&
-                      (q0[r].y - q0[r].w <= by1) && (q0[r].y + q0[r].w >= by0);
-            bal[r] = __ballot_sync(kFull, keep[r]);
-        }
-        float4 q1[R], q2[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-            if (keep[r]) {
-                q1[r] = __ldg(rp[r] + 1);  // (A, B, C, L)
-                q2[r] = __ldg(rp[r] + 2);  // (red, green, blue, 0)
+        for (int b = 0; b < BPW; ++b) {
+            const bool keep = row && !block_done(b) && (q.x - q.z <= bx1[b]) && (q.x + q.z >= bx0[b]);
+            const unsigned bal = __ballot_sync(kFull, keep);
+            if (keep) {
+                const int o = BPW * warp + b, k = __popc(bal & lt);
+                const float4* rp = a.rec + 3 * (int64_t)s;
+                cp_async(&sm.r.con[o][buf][k], rp + 1, 1);
+                cp_async(&sm.r.col[o][buf][k], rp + 2, 1);
+                sm.r.xy[o][buf][k] = make_float2(q.x, q.y);
             }
+            cnt[b] = __popc(bal);
+        }
+        cp_async_commit();
+    };
+    int s1 = load_slot(lane);
+    int s2 = load_slot(32 + lane), s3 = load_slot(64 + lane);
+    float4 q1 = load_cull(s1);
+    stage(s1, q1, 0);
+    q1 = load_cull(s2);
+    for (int base = 0, buf = 0; base < count; base += kRecStep, buf ^= 1) {
+        int now[BPW];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int j = base + CHUNK + 32 * r + lane;
-            if (j < last) {
-                rpn[r] = a.rec + 3 * (int64_t)slot_at(a, sk, first, j - first);
-                qn[r] = __ldg(rpn[r]);
+        for (int b = 0; b < BPW; ++b) now[b] = block_done(b) ? 0 : cnt[b];
+        stage(s2, q1, buf ^ 1);
+        s2 = s3;
+        q1 = load_cull(s3);
+        s3 = load_slot(base + 96 + lane);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        int n = now[0];
+        if (BPW > 1) {
+            __syncwarp();  // every lane's copies have landed: a done block's slots are overwritten
+            // fill the shorter list up with entries that change nothing (2^-1e30 = 0)
+            n = max(now[0], now[BPW - 1]);
+            const int mine = half ? now[BPW - 1] : now[0];
+            for (int k = mine + sub; k < n; k += LPB) {
+                sm.r.con[blk][buf][k] = make_float4(0.f, 0.f, 0.f, -1e30f);
+                sm.r.col[blk][buf][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                sm.r.xy[blk][buf][k] = make_float2(0.f, 0.f);
             }
         }
-        int below = 0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            if (keep[r]) {
-                const int k = below + __popc(bal[r] & lt);
-                sm.s[warp][k] = make_float4(q0[r].x, q1[r].x, q1[r].y, q1[r].w);
-                sm.q[warp][k] = make_float4(q0[r].y, q1[r].z, q2[r].x, q2[r].y);
-                sm.b[warp][k] = q2[r].z;
-            }
-            below += __popc(bal[r]);
-        }
-        __syncwarp();  // slot writes visible to the whole warp
-        const int cnt = below;
+        __syncwarp();  // this step's slots visible to the whole warp
 #pragma unroll 4
-        for (int k = 0; k < cnt; ++k) {
-            const float4 e = sm.s[warp][k];
-            const float4 q = sm.q[warp][k];
-            const float bl = sm.b[warp][k];
-            const float dx = cx - e.x;
-            const float adx2 = fmaf(e.y * dx, dx, e.w);  // A dx^2 + L
-            const float bdx = __fmul_rn(e.z, dx);  // kept apart from the fma below
-            const float dy0 = cy0 - q.x, dy1 = cy1 - q.x;
-            const float p0 = fmaf(fmaf(q.y, dy0, bdx), dy0, adx2);
-            const float p1 = fmaf(fmaf(q.y, dy1, bdx), dy1, adx2);
-            const f2 w = f2_mul(TT, f2_pack(ex2_approx(p0), ex2_approx(p1)));
-            float w0, w1;
-            f2_unpack(w, w0, w1);
-            R0 = fmaf(q.z, w0, R0);
-            R1 = fmaf(q.z, w1, R1);
-            G0 = fmaf(q.w, w0, G0);
-            G1 = fmaf(q.w, w1, G1);
-            B0 = fmaf(bl, w0, B0);
-            B1 = fmaf(bl, w1, B1);
-            TT = f2_sub(TT, w);
+        for (int k = 0; k < n; ++k) {
+            const float2 c = sm.r.xy[blk][buf][k];
+            const float4 e = sm.r.con[blk][buf][k];
+            const float4 q = sm.r.col[blk][buf][k];
+            const f2 dy = f2_sub(cy, f2_dup(c.y));
+            const f2 C = f2_dup(e.z), red = f2_dup(q.x), green = f2_dup(q.y), blue = f2_dup(q.z);
+#pragma unroll
+            for (int i = 0; i < BPW; ++i) {
+                const float dx = cx[i] - c.x;
+                const f2 adx2 = f2_dup(fmaf(__fmul_rn(e.x, dx), dx, e.w));  // A dx^2 + L
+                const f2 bdx = f2_dup(__fmul_rn(e.y, dx));
+                float p0, p1;
+                f2_unpack(f2_fma(f2_fma(C, dy, bdx), dy, adx2), p0, p1);
+                const f2 w = f2_mul(T[i], f2_pack(ex2_approx(p0), ex2_approx(p1)));
+                CR[i] = f2_fma(red, w, CR[i]);
+                CG[i] = f2_fma(green, w, CG[i]);
+                CB[i] = f2_fma(blue, w, CB[i]);
+                T[i] = f2_sub(T[i], w);
+            }
         }
-        __syncwarp();  // slots are rewritten by the next chunk
-        float T0, T1;
-        f2_unpack(TT, T0, T1);
-        done = T0 < tmin && T1 < tmin;
+        __syncwarp();  // this buffer is rewritten by the next step
+        if (CHUNK == kRecStep || (base & kRecStep) || base + kRecStep >= count) {
+            bool done = true;
+#pragma unroll
+            for (int c = 0; c < BPW; ++c) {
+                float t0, t1;
+                f2_unpack(T[c], t0, t1);
+                done = done && t0 < tmin && t1 < tmin;
+            }
+            donemask = __ballot_sync(kFull, done);
+        }
+        if (donemask == kFull) break;
     }
-    if (in0) store_pixel(v, px, py0, R0, G0, B0);
-    if (in1) store_pixel(v, px, py1, R1, G1, B1);
+    asm volatile("cp.async.wait_all;" ::: "memory");  // none in flight when the CTA goes on or ends
+#pragma unroll
+    for (int c = 0; c < BPW; ++c) {
+        if (px + c >= v.width) continue;
+        float r0, r1, g0, g1, b0, b1;
+        f2_unpack(CR[c], r0, r1);
+        f2_unpack(CG[c], g0, g1);
+        f2_unpack(CB[c], b0, b1);
+        if (iny0) store_pixel(v, px + c, py0, r0, g0, b0);
+        if (iny1) store_pixel(v, px + c, py1, r1, g1, b1);
+    }
 }
 
 // One CTA per tile, in the raster order (heavy tiles first) or of the view
 // group [tile_base, tile_base + grid).
 template <int TW, int TH, int CHUNK>
-__global__ void __launch_bounds__(TW * TH / 2, 2048 / (TW * TH)) raster_rec_kernel(RasterArgs a)
+__global__ void __launch_bounds__(RecShape<TW, TH>::NT, 640 / RecShape<TW, TH>::NT) raster_rec_kernel(RasterArgs a)
 {
-    __shared__ RecSmem<TW, TH, CHUNK> sm;
+    __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH>)];
+    RecSmem<TW, TH>& sm = *reinterpret_cast<RecSmem<TW, TH>*>(smem);
     const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[blockIdx.x]) : a.tile_base + (int64_t)blockIdx.x;
     raster_rec_tile<TW, TH, CHUNK>(a, gtile, sm);
 }
@@ -629,9 +712,11 @@ __global__ void __launch_bounds__(TW * TH / 2, 2048 / (TW * TH)) raster_rec_kern
 // an atomic queue over the raster order (heavy tiles first) until it runs
 // dry.
 template <int TW, int TH, int CHUNK>
-__global__ void __launch_bounds__(TW * TH / 2, 2048 / (TW * TH)) raster_rec_persistent_kernel(RasterArgs a)
+__global__ void __launch_bounds__(RecShape<TW, TH>::NT, 640 / RecShape<TW, TH>::NT)
+    raster_rec_persistent_kernel(RasterArgs a)
 {
-    __shared__ RecSmem<TW, TH, CHUNK> sm;
+    __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH>)];
+    RecSmem<TW, TH>& sm = *reinterpret_cast<RecSmem<TW, TH>*>(smem);
     __shared__ int64_t s_tile;
     for (;;) {
         if (threadIdx.x == 0) {
@@ -651,17 +736,18 @@ static void launch_rec(const RasterArgs& a, bool persistent, int num_sms, cudaSt
 {
     if (a.num_tiles_total <= 0) return;
     if (!persistent) {
-        raster_rec_kernel<TW, TH, CHUNK><<<(unsigned)a.num_tiles_total, TW * TH / 2, 0, st>>>(a);
+        raster_rec_kernel<TW, TH, CHUNK><<<(unsigned)a.num_tiles_total, RecShape<TW, TH>::NT, 0, st>>>(a);
         return;
     }
     static int per_sm = 0;  // same on every B200; queried once
     if (per_sm == 0) {
         int x = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x, raster_rec_persistent_kernel<TW, TH, CHUNK>, TW * TH / 2, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x, raster_rec_persistent_kernel<TW, TH, CHUNK>,
+                                                      RecShape<TW, TH>::NT, 0);
         per_sm = std::max(x, 1);
     }
     const int64_t grid = std::min<int64_t>((int64_t)per_sm * num_sms, a.num_tiles_total);
-    raster_rec_persistent_kernel<TW, TH, CHUNK><<<(unsigned)grid, TW * TH / 2, 0, st>>>(a);
+    raster_rec_persistent_kernel<TW, TH, CHUNK><<<(unsigned)grid, RecShape<TW, TH>::NT, 0, st>>>(a);
 }
 
 template <int TW, int TH>

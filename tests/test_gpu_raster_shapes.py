@@ -1,6 +1,8 @@
-"""The stage raster in reference mode on hand-made tile lists: batch
-remainders, image sizes that cut tiles, every tile shape, and entries whose
-exponent is not a number, against the oracle's raster of the same lists."""
+"""The rasters at the sizes where they can go wrong, against the oracle's
+raster of the same lists: the stage raster in reference mode on hand-made
+tile lists (batch remainders, image sizes that cut tiles, every tile shape,
+entries whose exponent is not a number) and the record raster of whole T_min
+frames."""
 import numpy as np
 import pytest
 
@@ -52,3 +54,34 @@ def test_reference_raster(gs, O, tile, size, wild):
     # one more for the truncation to 8 bits
     diff = np.abs(img.cpu().numpy().astype(int) - ref.astype(int))
     assert diff.max() <= 1, diff.max()
+
+
+@pytest.mark.parametrize("tile", [(16, 16), (16, 8), (8, 8)])
+@pytest.mark.parametrize("chunk", [32, 64])
+@pytest.mark.parametrize("n,size", [(1, (9, 5)), (40, (17, 16)), (700, (33, 47)), (9000, (50, 31))])
+def test_record_raster(gs, O, tile, chunk, n, size):
+    """Whole T_min frames whose blocks are cut by the image's edges, with one
+    entry up to a few thousand per tile, against the oracle's raster of the
+    frame's own lists and projected floats."""
+    import torch
+    W, H = size
+    sc = gs.scenes.uniform_scene(n, seed=n, log_scale_mu=-2.5)
+    rc = gs.RenderConfig(tile_w=tile[0], tile_h=tile[1], raster_chunk=chunk)
+    cam = gs.look_at((0.1, 0.2, 3.0), (0, 0, 0), (0, 1, 0), 50.0, W, H, 0.1, 100.0)
+    ctx = gs.Context(0)
+    scene = gs.Scene(ctx, sc["pos4"], sc["sr4"], gs.scenes.grouped_sh(sc["sh"]), 3)
+    f = lambda *s: torch.zeros(s, dtype=torch.float32, device="cuda")  # noqa: E731
+    xy, z, ell, conic, color = f(n, 2), f(n), f(n, 4), f(n, 4), f(n, 4)
+    img = torch.zeros((H, W, 4), dtype=torch.uint8, device="cuda")
+    gs.probe_frame(ctx, scene, [cam], rc, [img], xy, z, ell, conic, color)
+    h = lambda t: t.cpu().numpy()  # noqa: E731
+    keys, vals = O.build(h(xy), h(ell), h(z), cam, rc)
+    tiles = gs.num_tiles(W, H, rc)
+    keys, vals = O.sort(keys, vals, gs.key_bits(tiles))
+    ref = O.raster(cam, rc, O.ranges(keys, tiles), vals, h(xy), h(conic), h(color))
+    scene.close()
+    ctx.close()
+    # the image bar of this mode: the culled contributions are each below 2^-18
+    # and the stop below t_min, together within two 8-bit steps
+    diff = np.abs(h(img).astype(int) - ref.astype(int))
+    assert diff.max() <= 2, diff.max()
