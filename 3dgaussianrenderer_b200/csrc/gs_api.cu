@@ -113,14 +113,19 @@ struct Counters {
     unsigned long long raster_tile;                // persistent raster queue
     unsigned long long sort_tiles[kMaxPasses];     // onesweep tile queues
     unsigned long long scan_block;                 // tile scan block queue
-    unsigned long long slots;                      // (view, Gaussian) slots taken by the frame kernel
+    unsigned long long units;                      // units of large splats listed
+    unsigned long long unit_next;                  // and handed out
+    unsigned long long emit_batch;                 // bucket emission: overlap chunks handed out
+    unsigned long long slots;                      // frame kernel: (view, Gaussian) slots taken (low 32 bits) and
+                                                   // overlap chunks (high 32 bits)
     int64_t total;                                 // K
     int64_t sort_n;                                // min(K, key capacity)
     unsigned int big_tiles;                        // tiles sorted ahead of the raster (to 4096 keys)
     unsigned int huge_tiles;                       // those above 4096 keys
-    unsigned int order_heads[2];                   // raster order: heavy tiles placed, others placed
+    unsigned int class_tiles[kOrderClasses];       // raster order: tiles of each class, and
+    unsigned int class_heads[kOrderClasses];       // how many of them are placed
     int err;
-    int overflow;                                  // K > key capacity: the frame must be redone
+    int overflow;                                  // the key or overlap list was too short: redo the frame
     uint32_t epoch_scan, epoch_sort;               // look-back epochs of this frame
 };
 
@@ -215,7 +220,9 @@ struct gs_ctx {
     DevBuf keys0, vals0, keys1, vals1;     // tile lists
     DevBuf sort_hist, sort_status;
     DevBuf ranges;
-    DevBuf tile_count, cursor, big_list;   // tile-bucket ordering: keys per tile, bucket fill cursors, big tiles
+    DevBuf tile_count, big_list;           // tile-bucket ordering: keys per tile, big tiles
+    DevBuf overlaps, chunks;               // tile-bucket ordering: the frame's overlap list (BucketEmitArgs)
+    int64_t chunk_capacity = 0;
     DevBuf tile_order;                     // raster order of the tiles (heavy tiles first)
     DevBuf counters;
     DevBuf image;                          // images of the host-output variants
@@ -225,7 +232,6 @@ struct gs_ctx {
     int h_views_cap = 0;
     cudaEvent_t ev[8] = {};
     int64_t key_capacity = 0;
-    int64_t per_view_capacity = 0;         // Gaussians * views the splat buffers hold
     cudaStream_t cap_stream = nullptr;     // graph capture
     cudaStream_t copy_stream = nullptr;    // image read-back of the host-output batches
     cudaEvent_t ev_group[kMaxRasterGroups] = {};  // end of each raster view group
@@ -368,6 +374,28 @@ int ensure_key_buffers(gs_ctx* ctx, int64_t keys)
     return GS_OK;
 }
 
+// Grows the overlap list of tile-bucket frames to hold `chunks` chunks.
+int ensure_overlaps(gs_ctx* ctx, int64_t chunks)
+{
+    if (chunks <= ctx->chunk_capacity && ctx->overlaps.p) return GS_OK;
+    const size_t c = (size_t)std::max<int64_t>(chunks, 1);
+    ctx->chunk_capacity = 0;
+    if (ctx->overlaps.ensure(sizeof(uint2) * 32 * c) || ctx->chunks.ensure(sizeof(uint4) * c))
+        return fail(GS_ERR_OOM, "overlap list");
+    ctx->chunk_capacity = (int64_t)std::min(ctx->overlaps.bytes / (sizeof(uint2) * 32), ctx->chunks.bytes / sizeof(uint4));
+    return GS_OK;
+}
+
+// The raster's per-(view, Gaussian) inputs: records in T_min mode, the
+// reference's buffers otherwise (xy is the caller's, see both frame paths).
+int ensure_raster_inputs(gs_ctx* ctx, int termination, size_t items)
+{
+    const bool failed = termination == GS_TERM_TMIN
+                            ? ctx->rec.ensure(48 * items) != cudaSuccess
+                            : ctx->color.ensure(16 * items) != cudaSuccess || ctx->conic.ensure(16 * items) != cudaSuccess;
+    return failed ? fail(GS_ERR_OOM, "raster inputs") : GS_OK;
+}
+
 // One frame over `num_views` views of `scene` with GS_ORDER_ONESWEEP: keys
 // in Gaussian order at scanned offsets, radix sort, ranges.  The host reads
 // the exact key count between the projection and the emission.
@@ -403,16 +431,12 @@ int run_frame_onesweep(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams
     const int64_t chains = groups * num_views;
 
     // per-(view, Gaussian) buffers
-    if (items > ctx->per_view_capacity) {
-        const size_t m = (size_t)items;
-        if (ctx->color.ensure(16 * m) || ctx->xy.ensure(8 * m) || ctx->z.ensure(4 * m) || ctx->ell.ensure(16 * m) ||
-            ctx->conic.ensure(16 * m) || ctx->rect.ensure(8 * m) || ctx->offsets.ensure(4 * m) ||
-            ctx->rec.ensure(48 * m) || ctx->hitmask.ensure(4 * m)) {
-            ctx->per_view_capacity = 0;  // some of them were released: re-check them all next time
-            return fail(GS_ERR_OOM, "splat buffers");
-        }
-        ctx->per_view_capacity = items;
-    }
+    const size_t m = (size_t)std::max<int64_t>(items, 1);
+    if (ctx->xy.ensure(8 * m) || ctx->z.ensure(4 * m) || ctx->ell.ensure(16 * m) || ctx->rect.ensure(8 * m) ||
+        ctx->offsets.ensure(4 * m) || ctx->hitmask.ensure(4 * m))
+        return fail(GS_ERR_OOM, "splat buffers");
+    rc = ensure_raster_inputs(ctx, cfg.termination, m);
+    if (rc) return rc;
     if (sizeof(uint64_t) * (size_t)std::max<int64_t>(chains, 1) > ctx->scan_status.bytes) {
         if (ctx->scan_status.ensure(sizeof(uint64_t) * (size_t)std::max<int64_t>(chains, 1), true))
             return fail(GS_ERR_OOM, "scan status");
@@ -599,6 +623,8 @@ int plan_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams,
         p.tiles_total += (int64_t)vp.tiles_x * vp.tiles_y;
     }
     if (p.tiles_total >= (1ll << 31)) return fail(GS_ERR_INVALID, "too many tiles");
+    // the overlap list's tile ids; a view has at most 2^22 tiles
+    if (p.tiles_total >= (1ll << kOverlapTileBits)) return fail(kSplitViews, "more than 2^27 tiles");
     p.items = p.n * num_views;
     if (p.items >= (1ll << 31)) return fail(GS_ERR_INVALID, "views x Gaussians exceeds 2^31");
     p.groups = (p.n + 255) / 256;
@@ -606,16 +632,12 @@ int plan_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams,
     p.blocks = p.groups * ((num_views + p.vpb - 1) / p.vpb);
     p.deg = scene->sh_degree > 0 ? eval_degree(scene, cfg) : -1;
 
-    if (p.items > ctx->per_view_capacity) {
-        const size_t m = (size_t)p.items;
-        if (ctx->color.ensure(16 * m) || ctx->xy.ensure(8 * m) || ctx->z.ensure(4 * m) || ctx->ell.ensure(16 * m) ||
-            ctx->conic.ensure(16 * m) || ctx->rect.ensure(8 * m) || ctx->offsets.ensure(4 * m) ||
-            ctx->rec.ensure(48 * m) || ctx->hitmask.ensure(4 * m)) {
-            ctx->per_view_capacity = 0;  // some of them were released: re-check them all next time
-            return fail(GS_ERR_OOM, "splat buffers");
-        }
-        ctx->per_view_capacity = p.items;
-    }
+    const size_t m = (size_t)std::max<int64_t>(p.items, 1);
+    if (ctx->z.ensure(4 * m) || ctx->offsets.ensure(4 * m) || ctx->xy.ensure(8 * m) || ctx->ell.ensure(16 * m) ||
+        ctx->rect.ensure(8 * m))
+        return fail(GS_ERR_OOM, "splat buffers");
+    rc = ensure_raster_inputs(ctx, cfg.termination, m);
+    if (rc) return rc;
     const size_t tiles = (size_t)std::max<int64_t>(p.tiles_total, 1);
     const size_t scan_blocks = (tiles + kTileScanItems - 1) / kTileScanItems;
     if (sizeof(uint64_t) * scan_blocks > ctx->scan_status.bytes) {
@@ -623,7 +645,7 @@ int plan_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams,
     }
     if (sizeof(uint32_t) * tiles > ctx->tile_count.bytes) ctx->tile_count_dirty = true;
     if (ctx->ranges.ensure(sizeof(int32_t) * 2 * tiles) || ctx->tile_count.ensure(sizeof(uint32_t) * tiles) ||
-        ctx->cursor.ensure(sizeof(unsigned long long) * tiles) || ctx->big_list.ensure(sizeof(int32_t) * 2 * tiles) ||
+        ctx->big_list.ensure(sizeof(int32_t) * 2 * tiles) ||
         ctx->tile_order.ensure(sizeof(int32_t) * tiles))
         return fail(GS_ERR_OOM, "tile buffers");
     return GS_OK;
@@ -664,17 +686,23 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     fa.raster_mode = cfg.termination;
     fa.color = ctx->color.as<float4>();
     fa.xy = ctx->xy.as<float2>();
-    fa.z = ctx->z.as<float>();
     fa.ell = ctx->ell.as<float4>();
-    fa.conic = ctx->conic.as<float4>();
     fa.rect = ctx->rect.as<int2>();
+    fa.conic = ctx->conic.as<float4>();
     fa.rec = ctx->rec.as<float4>();
-    fa.hitmask = ctx->hitmask.as<uint32_t>();
     fa.offsets = ctx->offsets.as<int32_t>();  // slot -> view * n + i
+    fa.depth = ctx->z.as<uint32_t>();
     fa.err = &dc->err;
     fa.tile_count = ctx->tile_count.as<uint32_t>();
     fa.slot_counter = &dc->slots;
-    fa.aggregate = p.tiles_total <= kAggregateMaxTiles;
+    fa.overlaps = ctx->overlaps.as<uint2>();
+    fa.chunks = ctx->chunks.as<uint4>();
+    fa.chunk_capacity = ctx->chunk_capacity;
+    // the large splats' units live where only the tile sorts write later
+    fa.units = ctx->keys1.as<uint2>();
+    fa.unit_capacity = ctx->key_capacity;
+    fa.unit_count = &dc->units;
+    fa.unit_counter = &dc->unit_next;
     if (p.probe) {
         fa.probe_xy = reinterpret_cast<float2*>(p.probe->d_xy);
         fa.probe_z = p.probe->d_z;
@@ -682,12 +710,14 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
         fa.probe_conic = reinterpret_cast<float4*>(p.probe->d_conic);
         fa.probe_color = reinterpret_cast<float4*>(p.probe->d_color);
     }
-    if (p.n > 0) launch_frame_project(fa, p.deg, st, true);
+    if (p.n > 0) {
+        launch_frame_project(fa, p.deg, st, true);
+        launch_large_overlaps(fa, ctx->num_sms, st);
+    }
 
     TileScanArgs ta{};
     ta.count = ctx->tile_count.as<uint32_t>();
     ta.tiles = p.tiles_total;
-    ta.cursor = ctx->cursor.as<unsigned long long>();
     ta.ranges = ctx->ranges.as<int32_t>();
     ta.status = ctx->scan_status.as<uint64_t>();
     ta.block_counter = &dc->scan_block;
@@ -697,31 +727,38 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ta.capacity = ctx->key_capacity;
     ta.sort_n = &dc->sort_n;
     ta.overflow = &dc->overflow;
+    ta.slot_counter = &dc->slots;
+    ta.chunk_capacity = ctx->chunk_capacity;
+    ta.unit_count = &dc->units;
+    ta.unit_capacity = fa.unit_capacity;
     ta.big_list = ctx->big_list.as<int32_t>();
     ta.big_count = &dc->big_tiles;
     ta.huge_count = &dc->huge_tiles;
     ta.fused_cap = fused_tile_capacity(cfg.tile_w, cfg.tile_h);
+    ta.class_tiles = dc->class_tiles;
     launch_tile_scan(ta, st);
-    launch_tile_order(ctx->ranges.as<int32_t>(), p.tiles_total, &dc->total, ctx->tile_order.as<int32_t>(),
-                      dc->order_heads, st);
     GS_CUDA(record(ctx->ev[1], st, capturing));
     GS_CUDA(record(ctx->ev[2], st, capturing));
 
     BucketEmitArgs ea{};
-    ea.n = p.n;
-    ea.aggregate = p.tiles_total <= kAggregateMaxTiles;
-    ea.slot_count = &dc->slots;
-    ea.max_slots = p.items;
-    ea.views = ctx->views.as<ViewParams>();
-    ea.slot_gi = ctx->offsets.as<int32_t>();
-    ea.rect = ctx->rect.as<int2>();
-    ea.hitmask = ctx->hitmask.as<uint32_t>();
-    ea.xy = ctx->xy.as<float2>();
-    ea.ell = ctx->ell.as<float4>();
-    ea.z = ctx->z.as<float>();
-    ea.cursor = ctx->cursor.as<unsigned long long>();
+    ea.slot_counter = &dc->slots;
+    ea.overlaps = ctx->overlaps.as<uint2>();
+    ea.chunks = ctx->chunks.as<uint4>();
+    ea.chunk_capacity = ctx->chunk_capacity;
+    ea.depth = ctx->z.as<uint32_t>();
+    ea.ranges = ctx->ranges.as<int32_t>();
+    ea.tiles = p.tiles_total;
+    ea.overflow = &dc->overflow;
+    ea.err = &dc->err;
+    ea.big_count = &dc->big_tiles;
+    ea.huge_count = &dc->huge_tiles;
+    const bool in_groups = p.host_copy && p.host_copy->groups > 1 && cfg.termination == GS_TERM_TMIN;
+    const bool in_order = !in_groups && p.n > 0;
+    ea.order = in_order ? ctx->tile_order.as<int32_t>() : nullptr;
+    ea.class_tiles = dc->class_tiles;
+    ea.class_heads = dc->class_heads;
     ea.keys = ctx->keys0.as<uint64_t>();
-    ea.capacity = ctx->key_capacity;
+    ea.batch_counter = &dc->emit_batch;
     if (p.n > 0) launch_emit_bucket(ea, ctx->num_sms, st);
     GS_CUDA(record(ctx->ev[3], st, capturing));
 
@@ -757,15 +794,14 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ra.keys = ctx->keys0.as<uint64_t>();  // tiles up to the fused capacity are sorted by the raster CTA
     ra.slot_gi = ctx->offsets.as<int32_t>();
     ra.fused_cap = fused_tile_capacity(cfg.tile_w, cfg.tile_h);
-    ra.order = ctx->tile_order.as<int32_t>();
+    ra.order = ea.order;
     ra.rec_chunk = cfg.raster_chunk;
     ra.rec_persistent = cfg.raster_persistent;
     ra.sort_prefix_bits = cfg.sort_bits;
-    if (p.host_copy && p.host_copy->groups > 1 && ra.rec) {
+    if (in_groups) {
         // one launch per view group, in view order; a group's images are
         // complete at its event
         const HostCopy& hc = *p.host_copy;
-        ra.order = nullptr;
         for (int g = 0; g < hc.groups; ++g) {
             const int v0 = hc.first_view[g], v1 = hc.first_view[g + 1];
             const int64_t t0 = ctx->h_views[v0].tile_offset;
@@ -792,8 +828,8 @@ uint64_t layout_of(const gs_ctx* ctx)
 {
     const DevBuf* bufs[] = {&ctx->views, &ctx->color, &ctx->xy, &ctx->z, &ctx->ell, &ctx->conic, &ctx->rect,
                             &ctx->offsets, &ctx->rec, &ctx->hitmask, &ctx->scan_status, &ctx->keys0, &ctx->vals0,
-                            &ctx->keys1, &ctx->vals1, &ctx->ranges, &ctx->tile_count, &ctx->cursor, &ctx->big_list,
-                            &ctx->tile_order, &ctx->counters};
+                            &ctx->keys1, &ctx->vals1, &ctx->ranges, &ctx->tile_count, &ctx->big_list,
+                            &ctx->tile_order, &ctx->counters, &ctx->overlaps, &ctx->chunks};
     uint64_t h = 1469598103934665603ull;
     auto mix = [&h](uint64_t x) { h = (h ^ x) * 1099511628211ull; };
     for (const DevBuf* b : bufs) {
@@ -802,6 +838,7 @@ uint64_t layout_of(const gs_ctx* ctx)
     }
     mix((uint64_t)(uintptr_t)ctx->h_views);
     mix((uint64_t)ctx->key_capacity);
+    mix((uint64_t)ctx->chunk_capacity);
     return h;
 }
 
@@ -866,6 +903,9 @@ int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, 
         rc = ensure_key_buffers(ctx, std::max<int64_t>(p.items, 1 << 20));
         if (rc) return rc;
     }
+    // a first guess of three chunks per two warps and views; a frame that needs more is redone
+    rc = ensure_overlaps(ctx, std::max<int64_t>(p.items / 32 * 3 / 2, 1 << 15));
+    if (rc) return rc;
 
     // the graph slot of this frame, if any
     FrameGraph* g = nullptr;
@@ -940,15 +980,20 @@ int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, 
             return fail(kSplitViews, "more than 2^31 tile keys");
         }
         if (!ctx->h_counters->overflow) break;
-        if (attempts >= 2) return fail(GS_ERR_CUDA, "tile list overflow after regrowing");
+        if (attempts >= 3) return fail(GS_ERR_CUDA, "tile list overflow after regrowing");
         if (g) drop_graph(*g);
-        rc = ensure_key_buffers(ctx, std::min<int64_t>(K + K / 4, (1ll << 31) - 1));
+        // (the key and chunk counts are exact unless large splats' units did not fit)
+        const int64_t need = std::max(K > ctx->key_capacity ? K + K / 4 : 0, (int64_t)ctx->h_counters->units);
+        rc = ensure_key_buffers(ctx, std::min<int64_t>(need, (1ll << 31) - 1));
+        if (rc) return rc;
+        const int64_t chunks = (int64_t)(ctx->h_counters->slots >> 32);
+        rc = ensure_overlaps(ctx, chunks);
         if (rc) return rc;
     }
 
     ctx->last_tiles = p.tiles_total;
     ctx->last_keys = ctx->h_counters->total;
-    ctx->last_slots = (int64_t)ctx->h_counters->slots;
+    ctx->last_slots = (int64_t)(ctx->h_counters->slots & 0xFFFFFFFFull);
     ctx->last_fused_cap = fused_tile_capacity(cfg.tile_w, cfg.tile_h);
     if (stats) {
         stats->sh_eval_ms = 0.0;
@@ -959,11 +1004,11 @@ int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, 
         stats->total_ms = ms_between(ctx->ev[0], ctx->ev[5]);
         stats->num_keys = ctx->h_counters->total;
         stats->num_tiles = p.tiles_total;
-        // frame kernel, bucket emit, the two big-tile sorts; tile scan, tile order,
+        // frame kernel, large splats, bucket emit, the two big-tile sorts; tile scan,
         // raster (sorts the other tiles; one launch per view group when the
         // images stream to host memory group by group)
         const bool grouped = p.host_copy && p.host_copy->groups > 1 && cfg.termination == GS_TERM_TMIN;
-        stats->kernel_launches = (p.n > 0 ? 4 : 0) + 2 + (grouped ? p.host_copy->groups : 1);
+        stats->kernel_launches = (p.n > 0 ? 5 : 0) + 1 + (grouped ? p.host_copy->groups : 1);
         stats->graph_replay = replayed ? 1 : 0;
         stats->attempts = attempts;
     }
@@ -1232,8 +1277,8 @@ int gs_ctx_destroy(gs_ctx* ctx)
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     DevBuf* bufs[] = {&ctx->views, &ctx->color, &ctx->xy, &ctx->z, &ctx->ell, &ctx->conic, &ctx->rect,
                       &ctx->offsets, &ctx->rec, &ctx->hitmask, &ctx->scan_status, &ctx->view_stats, &ctx->keys0, &ctx->vals0, &ctx->keys1, &ctx->vals1,
-                      &ctx->sort_hist, &ctx->sort_status, &ctx->ranges, &ctx->tile_count, &ctx->cursor, &ctx->big_list, &ctx->tile_order,
-                      &ctx->counters, &ctx->image};
+                      &ctx->sort_hist, &ctx->sort_status, &ctx->ranges, &ctx->tile_count, &ctx->big_list, &ctx->tile_order,
+                      &ctx->overlaps, &ctx->chunks, &ctx->counters, &ctx->image};
     for (DevBuf* b : bufs) b->release();
     if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
     if (ctx->h_init) cudaFreeHost(ctx->h_init);
@@ -1251,8 +1296,8 @@ int64_t gs_ctx_device_bytes(const gs_ctx* ctx)
     if (!ctx) return 0;
     const DevBuf* bufs[] = {&ctx->views, &ctx->color, &ctx->xy, &ctx->z, &ctx->ell, &ctx->conic, &ctx->rect,
                             &ctx->offsets, &ctx->rec, &ctx->hitmask, &ctx->scan_status, &ctx->view_stats, &ctx->keys0, &ctx->vals0, &ctx->keys1, &ctx->vals1,
-                            &ctx->sort_hist, &ctx->sort_status, &ctx->ranges, &ctx->tile_count, &ctx->cursor, &ctx->big_list, &ctx->tile_order,
-                      &ctx->counters, &ctx->image};
+                            &ctx->sort_hist, &ctx->sort_status, &ctx->ranges, &ctx->tile_count, &ctx->big_list, &ctx->tile_order,
+                      &ctx->overlaps, &ctx->chunks, &ctx->counters, &ctx->image};
     int64_t t = 0;
     for (const DevBuf* b : bufs) t += (int64_t)b->bytes;
     return t;
@@ -1595,7 +1640,6 @@ int gs_stage_build(gs_ctx* ctx, int64_t n, const float* d_xy, const float* d_z, 
     const int64_t blocks = (n + 255) / 256;
     if (ctx->rect.ensure(8 * (size_t)n) || ctx->offsets.ensure(4 * (size_t)n) || ctx->hitmask.ensure(4 * (size_t)n))
         return fail(GS_ERR_OOM, "build buffers");
-    ctx->per_view_capacity = 0;  // rect/offsets may have been regrown: force the frame path to re-check
     ctx->last_tiles = -1;        // the last frame's slot indices are overwritten
     if (sizeof(uint64_t) * (size_t)blocks > ctx->scan_status.bytes) {
         if (ctx->scan_status.ensure(sizeof(uint64_t) * (size_t)blocks, true)) return fail(GS_ERR_OOM, "scan status");

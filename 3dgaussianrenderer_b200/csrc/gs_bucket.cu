@@ -7,7 +7,7 @@
 // kernel has already counted every tile's keys, so:
 //   1. tile scan   -- exclusive scan of the tile counts = each tile's range;
 //   2. bucket emit -- every overlap is written straight into its tile's
-//                     range, at a position claimed with one atomic, as
+//                     range, at the rank its count gave it, as
 //                     (depth << 32 | slot);
 //   3. tile sort   -- each tile's keys are ordered by depth in shared
 //                     memory (LSD radix over only the depth bits that vary
@@ -16,8 +16,8 @@
 //                     larger ones by a separate kernel.
 // The result per tile is exactly the order of a stable sort of the
 // reference's keys emitted in Gaussian order: depth first, index among equal
-// depths.  Each key crosses HBM about three times (emit, sort read, sorted
-// index write) instead of twice per radix pass.
+// depths.  Each key crosses HBM a few times (overlap list, emit, sort read)
+// instead of twice per radix pass.
 #include "gs_kernels.h"
 #include "gs_tilesort.cuh"
 
@@ -75,6 +75,17 @@ __device__ __forceinline__ uint64_t varying_bits_block(uint64_t or_v, uint64_t a
 
 }  // namespace
 
+// Raster order: tiles go to the rasteriser by falling key count, in classes of
+// half an octave (class 0 the heaviest), so that the longest CTAs start first
+// and the last wave is made of the shortest.
+__device__ __forceinline__ int order_class(const uint32_t count)
+{
+    if (count == 0) return kOrderClasses - 1;
+    const int l = 31 - __clz((int)count);
+    const int half = 2 * l + (l > 0 ? (int)((count >> (l - 1)) & 1u) : 0);
+    return kOrderClasses - 2 - min(half, kOrderClasses - 2);
+}
+
 // ---- 1. tile scan -------------------------------------------------------------
 
 __global__ void __launch_bounds__(kThreads) tile_scan_kernel(TileScanArgs a)
@@ -83,6 +94,8 @@ __global__ void __launch_bounds__(kThreads) tile_scan_kernel(TileScanArgs a)
     __shared__ int64_t s_tmp[kWarps];
     __shared__ int64_t s_base;
     __shared__ int64_t s_blk;
+    __shared__ unsigned int s_class[kOrderClasses];
+    if (threadIdx.x < kOrderClasses) s_class[threadIdx.x] = 0u;
     if (threadIdx.x == 0) s_blk = (int64_t)atomicAdd(a.block_counter, 1ull);
     __syncthreads();
     const int64_t blk = s_blk;
@@ -102,7 +115,10 @@ __global__ void __launch_bounds__(kThreads) tile_scan_kernel(TileScanArgs a)
     // leave the counts zeroed for the next frame (saves a clear per frame)
 #pragma unroll
     for (int j = 0; j < IPT; ++j)
-        if (first + j < a.tiles && c[j]) a.count[first + j] = 0u;
+        if (first + j < a.tiles) {
+            if (c[j]) a.count[first + j] = 0u;
+            atomicAdd(&s_class[order_class(c[j])], 1u);
+        }
     const int64_t excl = excl_scan_block(sum, s_tmp);
     if (threadIdx.x == kThreads - 1) {
         const uint64_t agg = (uint64_t)(excl + sum);
@@ -121,11 +137,13 @@ __global__ void __launch_bounds__(kThreads) tile_scan_kernel(TileScanArgs a)
             *a.total = total;
             if (a.sort_n) {
                 *a.sort_n = total < a.capacity ? total : a.capacity;
-                *a.overflow = total > a.capacity ? 1 : 0;
+                *a.overflow = total > a.capacity || (int64_t)(*a.slot_counter >> 32) > a.chunk_capacity ||
+                              (int64_t)*a.unit_count > a.unit_capacity;
             }
         }
     }
     __syncthreads();
+    if (threadIdx.x < kOrderClasses && s_class[threadIdx.x]) atomicAdd(&a.class_tiles[threadIdx.x], s_class[threadIdx.x]);
     int64_t run = s_base + excl;
     const int64_t cap = a.capacity;
 #pragma unroll
@@ -136,7 +154,6 @@ __global__ void __launch_bounds__(kThreads) tile_scan_kernel(TileScanArgs a)
                 a.big_list[a.tiles + atomicAdd(a.huge_count, 1u)] = (int32_t)t;
             else if (c[j] > (uint32_t)a.fused_cap)
                 a.big_list[atomicAdd(a.big_count, 1u)] = (int32_t)t;
-            a.cursor[t] = (unsigned long long)run;
             const int64_t lo = run < cap ? run : cap;
             const int64_t hi = run + c[j] < cap ? run + c[j] : cap;
             a.ranges[2 * t] = (int32_t)lo;
@@ -153,200 +170,104 @@ void launch_tile_scan(const TileScanArgs& a, cudaStream_t st)
     tile_scan_kernel<<<(unsigned)blocks, kThreads, 0, st>>>(a);
 }
 
-// ---- 1b. raster order of the tiles --------------------------------------------
-//
-// Tiles with more than 1.5x the average key count go first, so the longest
-// raster CTAs start in the first wave instead of stretching the last one;
-// the others follow (in reverse order, filled from the end).  One atomic
-// per warp and class.
-__global__ void __launch_bounds__(kThreads) tile_order_kernel(const int32_t* __restrict__ ranges, int64_t tiles,
-                                                             const int64_t* __restrict__ total,
-                                                             int32_t* __restrict__ order, unsigned int* heads)
-{
-    const int64_t t = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    const bool valid = t < tiles;
-    const int64_t cnt = valid ? (int64_t)(__ldg(&ranges[2 * t + 1]) - __ldg(&ranges[2 * t])) : 0;
-    const bool heavy = valid && 2 * cnt * tiles > 3 * *total;
-    const unsigned bh = __ballot_sync(kFull, heavy), bl = __ballot_sync(kFull, valid && !heavy);
-    const int lane = threadIdx.x & 31;
-    unsigned int h0 = 0, l0 = 0;
-    if (lane == 0) {
-        if (bh) h0 = atomicAdd(&heads[0], (unsigned)__popc(bh));
-        if (bl) l0 = atomicAdd(&heads[1], (unsigned)__popc(bl));
-    }
-    h0 = __shfl_sync(kFull, h0, 0);
-    l0 = __shfl_sync(kFull, l0, 0);
-    const unsigned below = lanemask_lt();
-    if (heavy)
-        order[h0 + __popc(bh & below)] = (int32_t)t;
-    else if (valid)
-        order[tiles - 1 - (int64_t)(l0 + __popc(bl & below))] = (int32_t)t;
-}
-
-void launch_tile_order(const int32_t* ranges, int64_t tiles, const int64_t* total, int32_t* order,
-                       unsigned int* heads, cudaStream_t st)
-{
-    if (tiles <= 0) return;
-    tile_order_kernel<<<(unsigned)((tiles + kThreads - 1) / kThreads), kThreads, 0, st>>>(ranges, tiles, total, order,
-                                                                                         heads);
-}
-
 // ---- 2. bucket emit -----------------------------------------------------------
-
-__device__ __forceinline__ uint32_t depth_bits(const float depth)
+//
+// The raster order of the tiles first (their classes' sizes are the scan's),
+// then one warp per chunk of the overlap list, four chunks in flight per warp.
+// Each place reads its overlap (8 bytes), its slot's depth and its tile's start
+// and writes one key; there is no chain longer than three loads.
+// The blocks (as many as fit) take batches of chunks in order from a counter:
+// a tile's next keys are then written close together in time and its sectors
+// leave L2 full, where a fixed stride lets fast blocks run ahead and sectors
+// are fetched and written back twice (4K view of 10M large splats, 337M keys:
+// 10.5 against 3.7 ms).  Before the list, the emission expanded each slot's
+// candidates, with an atomic per key and a second overlap test for large
+// splats: 12.5 ms there, 51 against 18 us on a 1080p view of 1M (1.8M keys),
+// 2.3 against 1.35 ms on 64 views of 3M (201M keys).  Counting a batch's
+// overlaps per tile in a shared-memory hash table, instead of taking the ranks
+// from the frame kernel's atomics, makes that kernel 0.4 ms faster there and
+// this one 1.6 ms slower.
+constexpr int kEmitUnroll = 4;
+constexpr int kEmitBlocksPerSm = 4;
+__global__ void __launch_bounds__(kThreads, kEmitBlocksPerSm) emit_bucket_kernel(BucketEmitArgs a)
 {
-    return (uint32_t)(make_key(0, depth) & 0xFFFFFFFFull);
-}
-
-// Called by the whole warp: each lane with `has` writes one key into tile
-// `gtile`'s bucket.  With `a.aggregate`, lanes of the same tile claim their
-// positions with one atomic (see warp_count_hits for when that pays); the
-// order inside a bucket is irrelevant, the tile sort orders it.
-__device__ __forceinline__ void put_keys(const BucketEmitArgs& a, const bool has, const int64_t gtile,
-                                         const uint32_t depth, const int64_t slot)
-{
-if (!a.aggregate) {
-        if (!has) return;
-        const unsigned long long pos = atomicAdd(&a.cursor[gtile], 1ull);
-        if ((int64_t)pos < a.capacity) a.keys[pos] = ((uint64_t)depth << 32) | (uint32_t)slot;
+    constexpr int U = kEmitUnroll;
+    constexpr int kBatch = kWarps * U;
+    __shared__ unsigned long long s_next[2];
+    if (*a.overflow || *a.err) {
+        // some list was too short, so keys of some tiles were never recorded,
+        // or the ranges are meaningless: the host redoes or drops the frame,
+        // and until then its tiles are empty
+        for (int64_t t = (int64_t)blockIdx.x * kThreads + threadIdx.x; t < 2 * a.tiles; t += (int64_t)gridDim.x * kThreads)
+            a.ranges[t] = 0;
+        for (int64_t t = (int64_t)blockIdx.x * kThreads + threadIdx.x; a.order && t < a.tiles; t += (int64_t)gridDim.x * kThreads)
+            a.order[t] = (int32_t)t;
+        if (blockIdx.x == 0 && threadIdx.x == 0) *a.big_count = *a.huge_count = 0u;
         return;
     }
-    const unsigned act = __ballot_sync(kFull, has);
-    if (!has) return;
-    const unsigned grp = __match_any_sync(act, (unsigned long long)gtile);
-    const int leader = __ffs(grp) - 1;
-    unsigned long long base = 0;
-    if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&a.cursor[gtile], (unsigned long long)__popc(grp));
-    base = __shfl_sync(grp, base, leader);
-    const unsigned long long pos = base + __popc(grp & lanemask_lt());
-    if ((int64_t)pos < a.capacity) a.keys[pos] = ((uint64_t)depth << 32) | (uint32_t)slot;
-}
-
-// Grid-strided over the slots in 256-slot steps (the slot count is only
-// known on the device).  Rectangles of at most 32 candidates expand the hit
-// mask the frame kernel recorded; larger ones are re-tested by the whole
-// warp, 32 candidates at a time.
-__global__ void __launch_bounds__(kThreads) emit_bucket_kernel(BucketEmitArgs a)
-{
-    const int64_t nslots = (int64_t)*a.slot_count;
-    const int lane = threadIdx.x & 31;
-    for (int64_t base = (int64_t)blockIdx.x * kThreads; base < nslots; base += (int64_t)gridDim.x * kThreads) {
-        const int64_t slot = base + threadIdx.x;
-        int cand = 0, view = 0;
-        int4 r = make_int4(0, 0, 0, 0);
-        Ell e = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        uint32_t depth = 0;
-        uint32_t m = 0;  // hit mask still to emit (rectangles of at most 32 candidates)
-        int64_t toff = 0;
-        int tiles_x = 0;
-        if (slot < nslots) {
-            // view * n + i < 2^31 (checked when the frame is planned): a
-            // 32-bit division
-            view = (int)((uint32_t)__ldg(&a.slot_gi[slot]) / (uint32_t)a.n);
-            r = unpack_rect(__ldg(&a.rect[slot]));
-            cand = rect_candidates(r);
-            depth = depth_bits(__ldg(&a.z[slot]));
-            if (cand <= 32) {
-                const ViewParams& v = a.views[view];
-                m = __ldg(&a.hitmask[slot]);
-                toff = v.tile_offset;
-                tiles_x = v.tiles_x;
-                cand = 0;
-            } else {
-                const float2 c = __ldg(&a.xy[slot]);
-                const float4 el = __ldg(&a.ell[slot]);
-                e = {c.x, c.y, el.x, el.y, el.z, el.w};
-            }
-        }
-        if (a.aggregate) {
-            // one overlap per lane and step, the warp converged
-            while (__any_sync(kFull, m != 0)) {
-                const bool has = m != 0;
-                int64_t gt = 0;
-                if (has) {
-                    const int c = __ffs(m) - 1;
-                    m &= m - 1;
-                    int cy, cx;
-                    divmod_small(c, r.z, cy, cx);
-                    gt = toff + (int64_t)(r.y + cy) * tiles_x + (r.x + cx);
-                }
-                put_keys(a, has, gt, depth, slot);
-            }
-        } else {
-            // up to 4 overlaps per step: their cursor atomics are in flight
-            // together, then the keys are written
-            const uint64_t lo = (uint32_t)slot;
-            while (m) {
-                int64_t gt[4];
-                unsigned long long pos[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    gt[u] = -1;
-                    if (m) {
-                        const int c = __ffs(m) - 1;
-                        m &= m - 1;
-                        int cy, cx;
-                        divmod_small(c, r.z, cy, cx);
-                        gt[u] = toff + (int64_t)(r.y + cy) * tiles_x + (r.x + cx);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (gt[u] >= 0) pos[u] = atomicAdd(&a.cursor[gt[u]], 1ull);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (gt[u] >= 0 && (int64_t)pos[u] < a.capacity) a.keys[pos[u]] = ((uint64_t)depth << 32) | lo;
-            }
-        }
-        if (__ballot_sync(kFull, cand > 0) == 0) continue;
-        // warp-cooperative walk over the large rectangles
-        int incl = cand;
+    const int64_t nchunks = (int64_t)(*a.slot_counter >> 32);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (a.order) {
+        static_assert(kOrderClasses == 32, "one class per lane");
+        int base = (int)a.class_tiles[lane];
+        const int mine = base;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += t;
+            const int t = __shfl_up_sync(kFull, base, o);
+            if (lane >= o) base += t;
         }
-        const int excl = incl - cand;
-        const int total = __shfl_sync(kFull, incl, 31);
-        for (int cb = 0; cb < total; cb += 32) {
-            const int c = cb + lane;
-            int o = 0;
+        base -= mine;  // tiles of the classes before this lane's
+        for (int64_t t0 = ((int64_t)blockIdx.x * kWarps + warp) * 32; t0 < a.tiles; t0 += (int64_t)gridDim.x * kThreads) {
+            const int64_t t = t0 + lane;
+            const bool valid = t < a.tiles;
+            const int cls = valid ? order_class((uint32_t)(a.ranges[2 * t + 1] - a.ranges[2 * t])) : kOrderClasses - 1;
+            const unsigned peers = __match_any_sync(kFull, valid ? cls : -1);
+            const int leader = __ffs(peers) - 1;
+            unsigned head = 0;
+            if (valid && lane == leader) head = atomicAdd(&a.class_heads[cls], (unsigned)__popc(peers));
+            head = __shfl_sync(kFull, head, leader);
+            const int at = __shfl_sync(kFull, base, cls) + (int)head + __popc(peers & lanemask_lt());
+            if (valid) a.order[at] = (int32_t)t;
+        }
+    }
+    if (threadIdx.x == 0) s_next[0] = atomicAdd(a.batch_counter, (unsigned long long)kBatch);
+    __syncthreads();
+    for (int it = 0;; it ^= 1) {
+        const int64_t c0 = (int64_t)s_next[it] + warp * U;
+        if ((int64_t)s_next[it] >= nchunks) return;
+        // the next batch is on its way while this one is written
+        if (threadIdx.x == 0) s_next[it ^ 1] = atomicAdd(a.batch_counter, (unsigned long long)kBatch);
+        uint4 h[U];
+        uint2 x[U];
+        uint32_t slot[U], depth[U];
+        int32_t lo[U];
 #pragma unroll
-            for (int b = 16; b >= 1; b >>= 1) {
-                const int t = __shfl_sync(kFull, incl, o + b - 1);
-                if (t <= c) o += b;
+        for (int u = 0; u < U; ++u) h[u] = c0 + u < nchunks ? __ldg(&a.chunks[c0 + u]) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if ((h[u].x >> lane) & 1u) x[u] = __ldcs(&a.overlaps[(c0 + u) * 32 + lane]);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if ((h[u].x >> lane) & 1u) {
+                const uint32_t owner = x[u].x >> kOverlapTileBits;
+                slot[u] = h[u].y + __popc(h[u].z & ((1u << owner) - 1u));
+                depth[u] = __ldg(&a.depth[slot[u]]);
+                lo[u] = a.ranges[2 * (int64_t)(x[u].x & ((1u << kOverlapTileBits) - 1u))];
             }
-            Ell oe;
-            oe.cx = __shfl_sync(kFull, e.cx, o);
-            oe.cy = __shfl_sync(kFull, e.cy, o);
-            oe.cs = __shfl_sync(kFull, e.cs, o);
-            oe.sn = __shfl_sync(kFull, e.sn, o);
-            oe.ex = __shfl_sync(kFull, e.ex, o);
-            oe.ey = __shfl_sync(kFull, e.ey, o);
-            int4 orr;
-            orr.x = __shfl_sync(kFull, r.x, o);
-            orr.y = __shfl_sync(kFull, r.y, o);
-            orr.z = __shfl_sync(kFull, r.z, o);
-            orr.w = __shfl_sync(kFull, r.w, o);
-            const int oexcl = __shfl_sync(kFull, excl, o);
-            const int oview = __shfl_sync(kFull, view, o);
-            const uint32_t od = __shfl_sync(kFull, depth, o);
-            bool hit = false;
-            int64_t gt = 0;
-            if (c < total) {
-                int tile = 0;
-                const ViewParams& v = a.views[oview];
-                hit = candidate_hit(oe, orr, c - oexcl, v, tile);
-                gt = v.tile_offset + tile;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if ((h[u].x >> lane) & 1u) {
+                a.keys[(int64_t)lo[u] + x[u].y] = ((uint64_t)depth[u] << 32) | slot[u];
             }
-            put_keys(a, hit, gt, od, base + (threadIdx.x & ~31) + o);
-        }
+        __syncthreads();
     }
 }
 
 void launch_emit_bucket(const BucketEmitArgs& a, int num_sms, cudaStream_t st)
 {
-    const int64_t blocks = std::min<int64_t>((a.max_slots + kThreads - 1) / kThreads, (int64_t)num_sms * 16);
+    const int64_t batch = kWarps * kEmitUnroll;
+    const int64_t work = std::max((a.chunk_capacity + batch - 1) / batch, (a.tiles + kThreads - 1) / kThreads);
+    const int64_t blocks = std::min<int64_t>(work, (int64_t)num_sms * kEmitBlocksPerSm);
     if (blocks <= 0) return;
     emit_bucket_kernel<<<(unsigned)blocks, kThreads, 0, st>>>(a);
 }

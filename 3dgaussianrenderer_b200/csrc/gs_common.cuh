@@ -620,6 +620,12 @@ __device__ __forceinline__ uint64_t make_key(const uint64_t tile, const float de
     return (tile << 32) | q;
 }
 
+// The key's depth half.
+__device__ __forceinline__ uint32_t depth_bits(const float depth)
+{
+    return (uint32_t)(make_key(0, depth) & 0xFFFFFFFFull);
+}
+
 // Packs a tile rectangle into 8 bytes (x0, y0 unsigned; w, h signed 16-bit).
 __device__ __forceinline__ int2 pack_rect(const int4 r)
 {

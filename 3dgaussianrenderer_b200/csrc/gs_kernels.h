@@ -61,6 +61,14 @@ inline int device_sm_count()
     return sms;
 }
 
+// Splats of more than kLargeCandidates candidate tiles are walked by
+// large_overlap_kernel, kUnitCandidates at a time (a threshold of 64 takes 7.2
+// instead of 8.0 ms for both kernels on the 4K view of 10M large splats, but
+// costs the warp walk the register that keeps its ballots: 0.4 ms on 64 views
+// of 3M).
+constexpr int kLargeCandidates = 32;
+constexpr int kUnitCandidates = 1024;
+
 // Fused SH + projection + count + scan over (view, Gaussian) pairs.  A block
 // owns one group of 256 Gaussians for `views_per_block` consecutive views;
 // every view has its own look-back chain over the groups, so offsets are
@@ -86,7 +94,7 @@ struct FrameArgs {
     float4* color;
     float2* xy;         // reference mode, or any mode when the rectangle has > 32 candidates
     float* z;
-    float4* ell;        // only when the rectangle has > 32 candidates
+    float4* ell;        // only when the rectangle has > 32 candidates (buckets: > kLargeCandidates, also rect)
     float4* conic;
     float4* rec;        // GS_TERM_TMIN raster record, 3 float4 per item (RasterRec)
     int2* rect;
@@ -98,14 +106,22 @@ struct FrameArgs {
     int64_t* view_total;  // [num_views] keys per view
     int* err;
     // tile-bucket pipeline (launch_frame_project with bucket = true): the
-    // (view, Gaussian) pairs that overlap a tile take slots from
-    // `slot_counter` in any order; every per-item output above is written
-    // at the slot instead of view * n + i, `offsets[slot]` receives
-    // view * n + caller index, and each overlapped tile's key count is added to
-    // tile_count[view tile offset + tile].
+    // (view, Gaussian) pairs with candidate tiles take slots in any order;
+    // every per-item output above is written at the slot instead of
+    // view * n + i, `offsets[slot]` receives view * n + caller index,
+    // `depth[slot]` the key's depth bits; tile_count[view tile offset + tile]
+    // counts the tile's keys and each overlap is recorded in the overlap list.
+    uint32_t* depth;
     uint32_t* tile_count;
-    unsigned long long* slot_counter;
-    int32_t aggregate;  // group same-tile count atomics of a warp (frames with few tiles)
+    unsigned long long* slot_counter;  // slots (low 32 bits) and overlap chunks (high) taken
+    uint2* overlaps;                   // [32 * chunk_capacity], see BucketEmitArgs
+    uint4* chunks;                     // [chunk_capacity]
+    int64_t chunk_capacity;
+    // splats of more than kLargeCandidates candidate tiles, in units
+    uint2* units;                      // [unit_capacity] (slot, unit of the splat)
+    unsigned long long* unit_count;    // units listed
+    unsigned long long* unit_counter;  // units handed out; zero at launch
+    int64_t unit_capacity;
     // probe outputs (diagnostics and tests; null in ordinary frames): the
     // projection of every Gaussian of every view at [view * n + caller
     // index] -- culled Gaussians as centre (-128, -128), depth -128, zero
@@ -117,37 +133,41 @@ struct FrameArgs {
     float4* probe_color;
 };
 
+// The overlap list of a tile-bucket frame, in chunks of 32 places.  Chunk c:
+//   chunks[c] = (mask of the places that hold an overlap, first slot of the
+//                warp that wrote it, its lanes that own a slot, -)
+//   overlaps[32 c + j] = (global tile | owner lane << kOverlapTileBits, rank in the tile)
+// The slot of an overlap is the first slot + the slot-owning lanes below the
+// owner.  A frame whose overlaps need more than chunk_capacity chunks is
+// flagged by the tile scan and redone.
+constexpr int kOverlapTileBits = 27;
+
 // Bucket emission: every overlap of slot s is written as
-// (depth bits << 32 | s) at an atomically claimed position of its tile's
-// bucket (cursor[tile], preset to the tile's first key by the tile scan).
+// (depth bits << 32 | s) at its rank in its tile's range.
 struct BucketEmitArgs {
-    int64_t n;                       // Gaussians per view
-    const unsigned long long* slot_count;
-    int64_t max_slots;               // grid bound
-    const ViewParams* views;
-    const int32_t* slot_gi;          // view * n + i of each slot
-    const int2* rect;
-    const uint32_t* hitmask;
-    const float2* xy;
-    const float4* ell;
-    const float* z;
-    unsigned long long* cursor;      // [tiles]
+    const unsigned long long* slot_counter;
+    const uint2* overlaps;
+    const uint4* chunks;
+    int64_t chunk_capacity;
+    const uint32_t* depth;           // [slots]
+    int32_t* ranges;                 // [2 * tiles]
+    int64_t tiles;
+    const int* overflow;             // either set: the frame does not stand; all ranges and the big-tile lists
+    const int* err;                  // are emptied
+    unsigned int* big_count;
+    unsigned int* huge_count;
+    int32_t* order;                  // [tiles] out: the raster order; null: not wanted
+    const unsigned int* class_tiles; // [kOrderClasses] tiles of each class (tile scan)
+    unsigned int* class_heads;       // [kOrderClasses] placed so far; zero at launch
     uint64_t* keys;
-    int64_t capacity;
-    int32_t aggregate;               // group same-tile cursor atomics of a warp (frames with few tiles)
+    unsigned long long* batch_counter;  // chunks handed out; zero at launch
 };
 
-// Frames of at most this many tiles (all views) group the same-tile atomics
-// of a warp in the frame kernel's counts and the bucket emission.
-constexpr int64_t kAggregateMaxTiles = 32768;
-
-// Exclusive scan of the per-tile key counts into tile ranges and bucket
-// cursors; the last block writes the key total.  Ranges are clamped to
+// Exclusive scan of the per-tile key counts into tile ranges; the last block writes the key total.  Ranges are clamped to
 // `capacity` (a frame whose keys do not fit is flagged, never overrun).
 struct TileScanArgs {
     uint32_t* count;                 // [tiles]; zeroed again after the scan
     int64_t tiles;
-    unsigned long long* cursor;      // [tiles] out: first key of the tile
     int32_t* ranges;                 // [2 * tiles] out: first, one past last
     uint64_t* status;                // look-back words, one per 4096 tiles
     unsigned long long* block_counter;
@@ -157,13 +177,19 @@ struct TileScanArgs {
     int64_t* total;                  // K
     int64_t capacity;
     int64_t* sort_n;                 // min(K, capacity)
-    int* overflow;                   // K > capacity
+    int* overflow;                   // K > capacity, or another list of the frame was too short
+    const unsigned long long* slot_counter;
+    int64_t chunk_capacity;
+    const unsigned long long* unit_count;  // of the large splats
+    int64_t unit_capacity;
     int32_t* big_list;               // out: [0, tiles) tiles with more than fused_cap keys, up to
                                      // kTileSortSmemKeys; [tiles, 2 tiles) the larger ones
     unsigned int* big_count;
     unsigned int* huge_count;
     int32_t fused_cap;
+    unsigned int* class_tiles;       // [kOrderClasses] tiles of each order class; zero at launch
 };
+constexpr int kOrderClasses = 32;
 
 // Per-tile sort of the buckets: each tile's keys are ordered by depth and,
 // among equal depths, by view * n + i, which is the order of a stable sort
@@ -276,12 +302,9 @@ void launch_project_stage(int64_t n, const float4* pos, const float4* sr, const 
                           float* z, float4* ell, float4* conic, cudaStream_t st);
 void launch_frame_project(const FrameArgs& a, int deg, cudaStream_t st, bool bucket = false);
 void launch_tile_scan(const TileScanArgs& a, cudaStream_t st);
-// Raster order of the tiles: those with more than 1.5x the average key count
-// (ranges and *total from the tile scan) first.  heads[2] start at zero.
-void launch_tile_order(const int32_t* ranges, int64_t tiles, const int64_t* total, int32_t* order,
-                       unsigned int* heads, cudaStream_t st);
 void launch_emit_bucket(const BucketEmitArgs& a, int num_sms, cudaStream_t st);
 void launch_tile_sort(const TileSortArgs& a, int num_sms, cudaStream_t st);
+void launch_large_overlaps(const FrameArgs& a, int num_sms, cudaStream_t st);
 void launch_count_stage(const FrameArgs& a, cudaStream_t st);
 // view_base[v] = sum of view_total[u < v]; *total = sum of all.  With a
 // non-null `sort_n`, also *sort_n = min(total, capacity) and *overflow = 1

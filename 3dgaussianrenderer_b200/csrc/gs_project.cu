@@ -92,13 +92,6 @@ __device__ __forceinline__ unsigned lane_range_mask(const int lo, const int hi)
 
 // Returns this lane's number of overlapping tiles; for rectangles of at
 // most 32 candidates also the hit mask (bit c = candidate c overlaps).
-// With a non-null `tile_count`, every overlap also adds one to its tile's
-// count (all lanes of the warp render the same view).  With `aggregate`,
-// lanes that hit the same tile in one step add their number with one atomic:
-// neighbouring Gaussians of a spatially ordered scene mostly share tiles,
-// and when a frame has few tiles, many atomics on one address serialise.
-// With many tiles the atomics spread out and the grouping costs more than
-// it saves.
 //
 // The overlap test is the reference's, in two phases: the walk decides every
 // candidate the cheap evaluation can call, and only if some candidate of the
@@ -128,81 +121,66 @@ __device__ __forceinline__ void add_hits(const unsigned bal, const WarpCands& w,
 // leaves out the owner's centre candidate oc0 (counted before the walk).
 __device__ __forceinline__ int walk_candidate(const int k, const int oc0) { return (oc0 >= 0 && k >= oc0) ? k + 1 : k; }
 
+// The tile holding a splat's centre is a hit (the centre test decides it):
+// each lane takes its own before the walk, which then leaves it out -- half
+// of the candidates on the benchmark's views.  The tile is found with the tile
+// rectangle's own arithmetic and confirmed with the centre test's; a centre on
+// a tile border falls through to the walk.  Returns the candidate index, -1
+// when there is none; sets the view-local tile.
+__device__ __forceinline__ int centre_candidate(const Ell& e, const int4 r, const int cand, const ViewParams& v,
+                                                int& tile0)
+{
+    if (cand <= 0) return -1;
+    const int gx = (int)floorf((e.cx + 1.0f) * 0.5f * v.tiles_xf);
+    const int gy = (int)floorf((e.cy + 1.0f) * 0.5f * v.tiles_yf);
+    const int lx = gx - r.x, ly = gy - r.y;
+    if (!(lx >= 0 && lx < r.z && ly >= 0 && ly < r.w && gx >= 0 && gx < v.tiles_x && gy >= 0 && gy < v.tiles_y)) return -1;
+    float x0, y0, x1, y1;
+    tile_clip_rect(v, gx, gy, x0, y0, x1, y1);
+    if (!(e.cx > x0 && e.cx < x1 && e.cy > y0 && e.cy < y1)) return -1;
+    tile0 = gy * v.tiles_x + gx;
+    return ly * r.z + lx;
+}
+
+// The owner's ellipse and rectangle, to the whole warp.
+__device__ __forceinline__ void owner_ell(const Ell& e, const int4 r, const int o, Ell& oe, int4& orr)
+{
+    oe.cx = __shfl_sync(kFull, e.cx, o);
+    oe.cy = __shfl_sync(kFull, e.cy, o);
+    oe.cs = __shfl_sync(kFull, e.cs, o);
+    oe.sn = __shfl_sync(kFull, e.sn, o);
+    oe.ex = __shfl_sync(kFull, e.ex, o);
+    oe.ey = __shfl_sync(kFull, e.ey, o);
+    orr.x = __shfl_sync(kFull, r.x, o);
+    orr.y = __shfl_sync(kFull, r.y, o);
+    orr.z = __shfl_sync(kFull, r.z, o);
+    orr.w = __shfl_sync(kFull, r.w, o);
+}
+
 __device__ __forceinline__ int warp_count_hits(const Ell& e, const int4 r, const int cand, const ViewParams& v,
-                                               uint32_t& mask, uint32_t* tile_count = nullptr,
-                                               const bool aggregate = false)
+                                               uint32_t& mask)
 {
     const int lane = threadIdx.x & 31;
-    // The tile holding the centre is a hit (the centre test decides it):
-    // each lane counts its own before the walk, which then leaves it out --
-    // half of the candidates on the benchmark's views.  The tile is found
-    // with the tile rectangle's own arithmetic and confirmed with the
-    // centre test's; a centre on a tile border falls through to the walk.
-    int c0 = -1, tile0 = 0;
-    if (cand > 0) {
-        const int gx = (int)floorf((e.cx + 1.0f) * 0.5f * v.tiles_xf);
-        const int gy = (int)floorf((e.cy + 1.0f) * 0.5f * v.tiles_yf);
-        const int lx = gx - r.x, ly = gy - r.y;
-        if (lx >= 0 && lx < r.z && ly >= 0 && ly < r.w && gx >= 0 && gx < v.tiles_x && gy >= 0 && gy < v.tiles_y) {
-            float x0, y0, x1, y1;
-            tile_clip_rect(v, gx, gy, x0, y0, x1, y1);
-            if (e.cx > x0 && e.cx < x1 && e.cy > y0 && e.cy < y1) {
-                c0 = ly * r.z + lx;
-                tile0 = gy * v.tiles_x + gx;
-            }
-        }
-    }
+    int tile0 = 0;
+    const int c0 = centre_candidate(e, r, cand, v, tile0);
     const bool pre = c0 >= 0;
     const WarpCands w = warp_scan_cands(cand - (pre ? 1 : 0));
     int hits = pre ? 1 : 0;
     mask = (pre && cand <= 32) ? (1u << c0) : 0u;
     bool undecided = false;
-    {
-        const unsigned bal = __ballot_sync(kFull, pre);
-        if (tile_count && pre) {
-            if (aggregate) {
-                const unsigned grp = __match_any_sync(bal, tile0);
-                if (lane == __ffs(grp) - 1) atomicAdd(&tile_count[v.tile_offset + tile0], (unsigned)__popc(grp));
-            } else {
-                atomicAdd(&tile_count[v.tile_offset + tile0], 1u);
-            }
-        }
-    }
-    auto owner_ell = [&](const int o, Ell& oe, int4& orr) {
-        oe.cx = __shfl_sync(kFull, e.cx, o);
-        oe.cy = __shfl_sync(kFull, e.cy, o);
-        oe.cs = __shfl_sync(kFull, e.cs, o);
-        oe.sn = __shfl_sync(kFull, e.sn, o);
-        oe.ex = __shfl_sync(kFull, e.ex, o);
-        oe.ey = __shfl_sync(kFull, e.ey, o);
-        orr.x = __shfl_sync(kFull, r.x, o);
-        orr.y = __shfl_sync(kFull, r.y, o);
-        orr.z = __shfl_sync(kFull, r.z, o);
-        orr.w = __shfl_sync(kFull, r.w, o);
-    };
     for (int base = 0; base < w.total; base += 32) {
         const int c = base + lane;
         const int o = owner_of(w.incl, c);
         Ell oe;
         int4 orr;
-        owner_ell(o, oe, orr);
+        owner_ell(e, r, o, oe, orr);
         const int oexcl = __shfl_sync(kFull, w.excl, o);
         const int oc0 = __shfl_sync(kFull, c0, o);
         int st = 0;
         int tile = 0;
         if (c < w.total) st = candidate_state(oe, orr, walk_candidate(c - oexcl, oc0), v, tile);
         undecided |= st < 0;
-        const bool hit = st > 0;
-        const unsigned bal = __ballot_sync(kFull, hit);
-        if (tile_count && hit) {
-            if (aggregate) {
-                const unsigned grp = __match_any_sync(bal, tile);
-                if (lane == __ffs(grp) - 1) atomicAdd(&tile_count[v.tile_offset + tile], (unsigned)__popc(grp));
-            } else {
-                atomicAdd(&tile_count[v.tile_offset + tile], 1u);
-            }
-        }
-        add_hits(bal, w, base, cand, c0, hits, mask);
+        add_hits(__ballot_sync(kFull, st > 0), w, base, cand, c0, hits, mask);
     }
     if (__any_sync(kFull, undecided)) {
         // rare: the candidates too close to call, in IEEE arithmetic
@@ -211,7 +189,7 @@ __device__ __forceinline__ int warp_count_hits(const Ell& e, const int4 r, const
             const int o = owner_of(w.incl, c);
             Ell oe;
             int4 orr;
-            owner_ell(o, oe, orr);
+            owner_ell(e, r, o, oe, orr);
             const int oexcl = __shfl_sync(kFull, w.excl, o);
             const int oc0 = __shfl_sync(kFull, c0, o);
             int tile = 0;
@@ -219,12 +197,241 @@ __device__ __forceinline__ int warp_count_hits(const Ell& e, const int4 r, const
             const int oc = walk_candidate(c - oexcl, oc0);
             if (c < w.total && candidate_state(oe, orr, oc, v, tile) < 0) hit = candidate_hit_ieee(oe, tile, v);
             const unsigned bal = __ballot_sync(kFull, hit);
-            if (!bal) continue;
-            if (tile_count && hit) atomicAdd(&tile_count[v.tile_offset + tile], 1u);
-            add_hits(bal, w, base, cand, c0, hits, mask);
+            if (bal) add_hits(bal, w, base, cand, c0, hits, mask);
         }
     }
     return hits;
+}
+
+// ---- overlaps of a warp's Gaussians, for the tile buckets -------------------------
+//
+// The same walk, but every overlap is recorded once and for all: one atomic on
+// its tile's key count returns its rank in the tile, and (tile, owner lane,
+// rank) goes to the overlap list in chunks of 32 (BucketEmitArgs).  The bucket
+// emission then needs neither another overlap test nor atomics.  An atomic's
+// result is used one step of the walk later, so its latency overlaps the next
+// step's tests.
+//
+// Every lane with candidates takes a slot; slots and chunks come from one
+// 64-bit atomic per warp (slots in the low half): a chunk for the centre tiles
+// and one per step of the walk, the step's ballot being its mask.  Splats of
+// more than kLargeCandidates candidates are left to large_overlap_kernel, so a
+// walk has at most 32 steps and lane s keeps step s's ballot until the chunks
+// are written.  The walk's registers bound the frame kernel (64 per thread):
+// what the lanes exchange is packed.
+
+// A warp's walk before its first step; the slots and chunks and the centre
+// tiles' ranks are on their way.
+struct BucketWalk {
+    int incl;                // inclusive scan of the lanes' candidates but the centre
+    int total;
+    int own;                 // (exclusive scan << 8 | centre candidate + 1) of this lane
+    unsigned preb;           // lanes with a centre tile
+    unsigned long long got;  // lane 0: (first chunk << 32 | first slot)
+};
+
+// Overlaps recorded but not yet written, because their ranks (and for the
+// first ones their chunk) are on their way: lanes with `has` write (where, rank
+// of lane `from` + more).
+struct OverlapPending {
+    uint32_t where;  // tile | owner << kOverlapTileBits
+    uint32_t rank;
+    int from, more;
+    bool has;
+};
+
+__device__ __forceinline__ void write_pending(const FrameArgs& a, const OverlapPending& x, const uint32_t chunk)
+{
+    const uint32_t rank = __shfl_sync(kFull, x.rank, x.from) + (uint32_t)x.more;
+    // chunks past the list's end are dropped: the frame is redone with a longer one
+    if (x.has && chunk < a.chunk_capacity)
+        a.overlaps[(int64_t)chunk * 32 + (threadIdx.x & 31)] = make_uint2(x.where, rank);
+}
+
+// The candidate of this lane in step `s` of the walk: 1 hit, 0 miss, -1 too
+// close to call; sets its owner, the owner's ellipse and the view-local tile.
+__device__ __forceinline__ int walk_step(const Ell& e, const int2 pr, const BucketWalk& k, const int s, const ViewParams& v,
+                                         Ell& oe, int& o, int& tile)
+{
+    const int c = 32 * s + (int)(threadIdx.x & 31);
+    o = owner_of(k.incl, c);
+    oe.cx = __shfl_sync(kFull, e.cx, o);
+    oe.cy = __shfl_sync(kFull, e.cy, o);
+    oe.cs = __shfl_sync(kFull, e.cs, o);
+    oe.sn = __shfl_sync(kFull, e.sn, o);
+    oe.ex = __shfl_sync(kFull, e.ex, o);
+    oe.ey = __shfl_sync(kFull, e.ey, o);
+    int2 opr;
+    opr.x = __shfl_sync(kFull, pr.x, o);
+    opr.y = __shfl_sync(kFull, pr.y, o);
+    const int own = __shfl_sync(kFull, k.own, o);
+    tile = 0;
+    if (c >= k.total) return 0;
+    return candidate_state(oe, unpack_rect(opr), walk_candidate(c - (own >> 8), (own & 0xFF) - 1), v, tile);
+}
+
+// Sets up the walk over the candidates (cand, 0 for lanes that take no part)
+// of a warp whose lanes in `owners` take slots, and counts the centre tiles.
+__device__ __forceinline__ BucketWalk start_walk(const Ell& e, const int4 r, const int cand, const ViewParams& v,
+                                                 const FrameArgs& a, const unsigned owners, OverlapPending& x)
+{
+    const int lane = threadIdx.x & 31;
+    BucketWalk k;
+    int tile0 = 0;
+    const int c0 = centre_candidate(e, r, cand, v, tile0);
+    x.has = c0 >= 0;
+    k.preb = __ballot_sync(kFull, x.has);
+    const WarpCands w = warp_scan_cands(cand - (x.has ? 1 : 0));
+    k.incl = w.incl;
+    k.total = w.total;
+    k.own = (w.excl << 8) | (c0 + 1);
+    k.got = 0;
+    if (lane == 0)
+        k.got = atomicAdd(a.slot_counter, ((unsigned long long)((k.preb ? 1 : 0) + ((w.total + 31) >> 5)) << 32) |
+                                              (unsigned long long)__popc(owners));
+    // neighbours in the scene's order mostly share their centre tile: one
+    // atomic per tile and warp (1024x1024 view of 3M: frame kernel -14 %)
+    x.where = ((uint32_t)v.tile_offset + (uint32_t)tile0) | ((uint32_t)lane << kOverlapTileBits);
+    x.rank = 0;
+    x.from = lane;
+    x.more = 0;
+    if (x.has) {
+        const unsigned grp = __match_any_sync(k.preb, tile0);
+        x.from = __ffs(grp) - 1;
+        x.more = __popc(grp & lanemask_lt());
+        if (lane == x.from) x.rank = atomicAdd(&a.tile_count[v.tile_offset + tile0], (unsigned)__popc(grp));
+    }
+    return k;
+}
+
+// The walk.  Leaves the overlaps of its last step (or of the centre tiles) in
+// `x`, to be written to chunk `last`.  With `track`, returns the lanes that own
+// an overlap.
+__device__ __forceinline__ unsigned run_walk(const Ell& e, const int2 pr, const ViewParams& v, const FrameArgs& a,
+                                             const BucketWalk& k, const bool track, OverlapPending& x, unsigned& mine)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t toff = (uint32_t)v.tile_offset;
+    const int steps = (k.total + 31) >> 5;
+    unsigned reached = k.preb;
+    uint32_t chunk = 0;  // of the pending overlaps
+    bool undecided = false;
+    mine = 0;
+    for (int s = 0; s < steps; ++s) {
+        int o, tile;
+        Ell oe;
+        const int st = walk_step(e, pr, k, s, v, oe, o, tile);
+        undecided |= st < 0;
+        const bool hit = st > 0;
+        const unsigned bal = __ballot_sync(kFull, hit);
+        if (lane == s) mine = bal;
+        if (track) reached |= __reduce_or_sync(kFull, hit ? 1u << o : 0u);
+        uint32_t rank = 0;
+        if (hit) rank = atomicAdd(&a.tile_count[toff + (uint32_t)tile], 1u);
+        if (s == 0) chunk = (uint32_t)(__shfl_sync(kFull, k.got, 0) >> 32);
+        if (s > 0 || k.preb) write_pending(a, x, chunk++);
+        x = {(toff + (uint32_t)tile) | ((uint32_t)o << kOverlapTileBits), rank, lane, 0, hit};
+    }
+    if (__any_sync(kFull, undecided)) {
+        // rare: the candidates too close to call, in IEEE arithmetic
+        write_pending(a, x, chunk);
+        x.has = false;
+        const uint32_t chunk0 = chunk - (uint32_t)(steps - 1);
+        for (int s = 0; s < steps; ++s) {
+            int o, tile;
+            Ell oe;
+            bool hit = walk_step(e, pr, k, s, v, oe, o, tile) < 0;
+            if (!__any_sync(kFull, hit)) continue;
+            if (hit) hit = candidate_hit_ieee(oe, tile, v);
+            const unsigned bal = __ballot_sync(kFull, hit);
+            if (lane == s) mine |= bal;
+            if (track) reached |= __reduce_or_sync(kFull, hit ? 1u << o : 0u);
+            OverlapPending y = {(toff + (uint32_t)tile) | ((uint32_t)o << kOverlapTileBits), 0u, lane, 0, hit};
+            if (hit) y.rank = atomicAdd(&a.tile_count[toff + (uint32_t)tile], 1u);
+            write_pending(a, y, chunk0 + (uint32_t)s);
+        }
+    }
+    return reached;
+}
+
+// ---- large splats -----------------------------------------------------------------
+//
+// A splat that covers hundreds of tiles would hold its warp, and its block,
+// while the rest of the frame is long done: on a 4K view of 10M large splats the
+// frame kernel spent 60 % of its time in the few blocks next to the camera.
+// Splats of more than kLargeCandidates candidates keep their ellipse and
+// rectangle at their slot and are listed, their candidates cut into units of
+// kUnitCandidates; large_overlap_kernel takes one unit per warp, from a
+// counter.  The threshold is about where a splat fills whole steps of a warp
+// of its own.
+
+// Lists the units of this warp's large splats.
+__device__ __forceinline__ void list_large(const int cand, const bool large, const uint32_t slot, const FrameArgs& a)
+{
+    const int units = large ? (cand + kUnitCandidates - 1) / kUnitCandidates : 0;
+    const WarpCands w = warp_scan_cands(units);
+    unsigned long long got = 0;
+    if ((threadIdx.x & 31) == 0) got = atomicAdd(a.unit_count, (unsigned long long)w.total);
+    const int64_t u0 = (int64_t)__shfl_sync(kFull, got, 0) + w.excl;
+    for (int u = 0; u < units; ++u)
+        if (u0 + u < a.unit_capacity) a.units[u0 + u] = make_uint2(slot, (uint32_t)u);
+}
+
+// One unit per warp: its overlaps' ballots first (step s's in lane s), then
+// exactly as many chunks as they fill, then the ranks and the list entries.
+__global__ void __launch_bounds__(256) large_overlap_kernel(const __grid_constant__ FrameArgs a)
+{
+    static_assert(kUnitCandidates == 1024, "one step of a unit per lane");
+    const int lane = threadIdx.x & 31;
+    int64_t units = (int64_t)*a.unit_count;
+    if (units > a.unit_capacity) units = a.unit_capacity;
+    if (units == 0) return;
+    unsigned long long next = 0;
+    if (lane == 0) next = atomicAdd(a.unit_counter, 1ull);
+    for (;;) {
+        const int64_t k = (int64_t)__shfl_sync(kFull, next, 0);
+        if (k >= units) return;
+        if (lane == 0) next = atomicAdd(a.unit_counter, 1ull);  // on its way while this unit is walked
+        const uint2 unit = __ldg(&a.units[k]);
+        const uint32_t slot = unit.x;
+        const float2 centre = __ldg(&a.xy[slot]);
+        const float4 el = __ldg(&a.ell[slot]);
+        const Ell e = {centre.x, centre.y, el.x, el.y, el.z, el.w};
+        const int4 r = unpack_rect(__ldg(&a.rect[slot]));
+        const ViewParams& v = a.views[(uint32_t)__ldg(&a.offsets[slot]) / (uint32_t)a.n];
+        const int c0 = (int)unit.y * kUnitCandidates;
+        const int total = min(rect_candidates(r) - c0, kUnitCandidates);
+        const int steps = (total + 31) >> 5;
+        unsigned mine = 0;
+        for (int s = 0; s < steps; ++s) {
+            const int c = 32 * s + lane;
+            int tile;
+            const bool hit = c < total && candidate_hit(e, r, c0 + c, v, tile);
+            const unsigned bal = __ballot_sync(kFull, hit);
+            if (lane == s) mine = bal;
+        }
+        const WarpCands w = warp_scan_cands(__popc(mine));
+        if (w.total == 0) continue;
+        const int chunks = (w.total + 31) >> 5;
+        unsigned long long got = 0;
+        if (lane == 0) got = atomicAdd(a.slot_counter, (unsigned long long)chunks << 32);
+        const int64_t first = (int64_t)(__shfl_sync(kFull, got, 0) >> 32);
+        const bool room = first + chunks <= a.chunk_capacity;
+        if (room && lane < chunks) {
+            const int left = w.total - 32 * lane;
+            a.chunks[first + lane] = make_uint4(left >= 32 ? kFull : (1u << left) - 1u, slot, 0u, 0u);
+        }
+        for (int s = 0; s < steps; ++s) {
+            const unsigned bal = __shfl_sync(kFull, mine, s);
+            const int at = __shfl_sync(kFull, w.excl, s);
+            if (!((bal >> lane) & 1u)) continue;
+            int lx, ly;
+            divmod_small(c0 + 32 * s + lane, r.z, ly, lx);
+            const uint32_t gt = (uint32_t)v.tile_offset + (uint32_t)((r.y + ly) * v.tiles_x + r.x + lx);
+            const uint32_t rank = atomicAdd(&a.tile_count[gt], 1u);
+            if (room) a.overlaps[first * 32 + at + __popc(bal & lanemask_lt())] = make_uint2(gt, rank);
+        }
+    }
 }
 
 // ---- block scan + decoupled look-back along one chain ---------------------------
@@ -288,122 +495,209 @@ __device__ __forceinline__ int64_t acquire_tile(unsigned long long* counter)
 // [c*vpb, (c+1)*vpb), c = tile / groups.  It reads position and
 // scale/rotation of its 256 Gaussians once and, for SH scenes, brings the
 // group's coefficients (the first 3*(DEG+1)^2 rows of the grouped layout,
-// contiguous) into shared memory with one TMA bulk copy.  Then per view:
+// contiguous) into shared memory with one TMA bulk copy, once a view shows one
+// of them.  Then per view:
 // SH colour, projection, tile rectangle, exact overlap count, and the
 // within-view key offset from that view's look-back chain.  Gaussians that
 // overlap no tile write only their offset.
 //
-// BUCKET: no scan at all -- each overlapping (view, Gaussian) takes a slot
-// (one atomic per warp) and adds its overlaps to the per-tile counts; the
-// blocks are independent and run in launch order.
+// BUCKET: no scan at all -- each (view, Gaussian) with candidate tiles takes a
+// slot and its overlaps go to the overlap list with their ranks in their
+// tiles (warp_bucket_hits); the blocks are independent and run in launch order.
+__device__ __forceinline__ void sh_wait(uint64_t* bar, int* err)
+{
+    int spins = 0;
+    while (!mbar_try_wait(bar, 0)) {
+        if (++spins > kSpinLimit) {
+            // a bulk copy from valid device memory always lands; report and
+            // carry on (the frame is discarded by the host)
+            atomicCAS(err, 0, kErrTimeout);
+            return;
+        }
+    }
+}
+
+// A load the compiler may not keep in registers across the views.
+__device__ __forceinline__ float4 reload(const float4* p)
+{
+    float4 x;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+                 : "l"(p));
+    return x;
+}
+
+// The T_min raster record of a splat: centre from e, conic in (g.x, g.y, g.z).
+__device__ __forceinline__ void write_record(float4* rec, const Ell& e, const float4 g, const float4 col)
+{
+    float ex, ey, A = -0.72134752f * g.x, B = -1.44269504f * g.y, C = -0.72134752f * g.z;
+    float L = lg2_approx(col.w);
+    const float det = g.x * g.z - g.y * g.y;
+    if (!(det > 0.0f) || !(g.x > 0.0f) || !(g.z > 0.0f) || !(col.w > kCullAlpha)) {
+        // contributes nothing anywhere: alpha below the cutoff, or a conic
+        // that is not positive definite
+        ex = ey = -1e30f;
+        A = B = C = 0.0f;
+        L = -1e30f;
+    } else {
+        // qc = 2 ln(opacity / cutoff) = 2 ln 2 (L + 18); 1.0001 covers the
+        // approximations
+        const float qc = 1.38643f * (L + 18.0f);
+        const float rdet = rcp_approx(det);
+        ex = sqrt_approx(qc * g.z * rdet);
+        ey = sqrt_approx(qc * g.x * rdet);
+    }
+    rec[0] = make_float4(e.cx, e.cy, ex, ey);
+    rec[1] = make_float4(A, B, C, L);
+    rec[2] = make_float4(col.x, col.y, col.z, 0.0f);
+}
+
+// MANY: a block draws several views.  It then keeps its Gaussians' attributes
+// in registers and waits for their coefficients once, before the first view;
+// with one view the attributes are read again after the walk, which needs the
+// registers, and the copy is asked for only where a Gaussian is in view and
+// overlaps the walk (1080p view of 1M: 104 against 112 us; 64 views of 3M: 6.3
+// against 6.6 ms).
 // Blocks per SM: 4 (64 registers); the exact projection at SH degree 3
 // keeps 80 registers (3 blocks)
-template <int DEG, bool BUCKET, bool FAST>
-__global__ void __launch_bounds__(256, (DEG >= 3 && !FAST) ? 3 : 4) frame_project_kernel(FrameArgs a)
+template <int DEG, bool BUCKET, bool FAST, bool MANY>
+__global__ void __launch_bounds__(256, (DEG >= 3 && !FAST) ? 3 : 4) frame_project_kernel(const __grid_constant__ FrameArgs a)
 {
     extern __shared__ __align__(128) float s_sh[];  // [3*(DEG+1)^2][256]
     __shared__ __align__(8) uint64_t s_bar;
+    __shared__ float4 s_geom[BUCKET ? 256 : 1];  // conic and depth across the walk
     const int64_t tile = BUCKET ? (int64_t)blockIdx.x : acquire_tile(a.tile_counter);
     const int64_t chunk = tile / a.groups;
     const int64_t group = tile - chunk * a.groups;
-    const int64_t i = group * 256 + threadIdx.x;
+    const int i = (int)group * 256 + (int)threadIdx.x;  // n < 2^31
     const bool valid = i < a.n;
     const int v0 = (int)chunk * a.views_per_block;
     const int v1 = min(a.num_views, v0 + a.views_per_block);
     const uint32_t epoch = a.epoch_dev ? *a.epoch_dev : a.epoch;
     constexpr int NCOEF = DEG >= 0 ? 3 * (DEG + 1) * (DEG + 1) : 0;
+    const int at = valid ? i : 0;  // where this thread's loads go
+    int gid = i;  // the Gaussian's caller index: equal depths are ordered by it
+    if (BUCKET && a.orig) gid = __ldg(&a.orig[at]);
 
-    if (DEG >= 0) {
-        if (threadIdx.x == 0) {
-            mbar_init(&s_bar, 1);
-            bulk_load(s_sh, a.sh + group * 256 * (int64_t)a.sh_count, NCOEF * 256 * sizeof(float), &s_bar);
+    if (DEG >= 0 && threadIdx.x == 0) mbar_init(&s_bar, 1);
+    bool sh_asked = DEG < 0 || MANY;  // the coefficients' copy has started (block-uniform) ...
+    bool sh_here = sh_asked;          // ... and, as this thread knows, landed
+    auto ask_sh = [&] {
+        bulk_load(s_sh, a.sh + group * 256 * (int64_t)a.sh_count, NCOEF * 256 * sizeof(float), &s_bar);
+    };
+    float4 kept_p = make_float4(0.f, 0.f, 0.f, 0.f), kept_sr = kept_p;
+    if (MANY) {
+        if (DEG >= 0 && threadIdx.x == 0) ask_sh();
+        kept_p = __ldg(&a.pos[at]);
+        kept_sr = __ldg(&a.sr[at]);
+        if (DEG >= 0) {
+            __syncthreads();  // barrier initialised before anyone polls it
+            sh_wait(&s_bar, a.err);
         }
     }
-    float4 p = make_float4(0.f, 0.f, 0.f, 0.f), sr = p, cin = p;
-    int64_t gid = i;  // the Gaussian's caller index: equal depths are ordered by it
-    if (valid) {
-        if (BUCKET && a.orig) gid = __ldg(&a.orig[i]);
-        p = __ldg(&a.pos[i]);
-        sr = __ldg(&a.sr[i]);
-        if (DEG < 0) cin = __ldg(&a.color_in[i]);
-    }
-    if (DEG >= 0) {
-        __syncthreads();  // barrier initialised before anyone polls it
-        int spins = 0;
-        while (!mbar_try_wait(&s_bar, 0)) {
-            if (++spins > kSpinLimit) {
-                // a bulk copy from valid device memory always lands; report
-                // and carry on (the frame is discarded by the host)
-                if (threadIdx.x == 0) atomicCAS(a.err, 0, kErrTimeout);
-                break;
-            }
-        }
-    }
+
+    // the colour towards view v: of the model, or from the coefficients
+    auto colour = [&](const ViewParams& v) {
+        if (DEG < 0) return reload(&a.color_in[at]);
+        if (!sh_here) sh_wait(&s_bar, a.err);
+        sh_here = true;
+        const float4 p = MANY ? kept_p : reload(&a.pos[at]);
+        const float3 d = view_dir(v, p);
+        const float3 c = sh_color<(DEG < 0 ? 0 : DEG), false>(d.x, d.y, d.z, s_sh + threadIdx.x, 256);
+        return make_float4(c.x, c.y, c.z, p.w);
+    };
 
     for (int view = v0; view < v1; ++view) {
         const ViewParams& v = a.views[view];
-        const int64_t o = (int64_t)view * a.n + i;
         Ell e = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         int4 r = make_int4(0, 0, 0, 0);
         int cand = 0;
         Splat s;
-        float4 col = cin;
         bool projected = false;
         if (valid) {
             // outside the frustum: culled, no tile (whole warps of a
             // spatially ordered scene skip the projection together)
+            const float4 p = MANY ? kept_p : reload(&a.pos[at]);
             const ViewPos w = view_position<FAST>(p, v);
             if (in_frustum(w)) {
                 projected = true;
-                s = project_gaussian<FAST>(w, sr, v);
+                s = project_gaussian<FAST>(w, MANY ? kept_sr : reload(&a.sr[at]), v);
                 e = {s.x, s.y, s.cs, s.sn, s.ex, s.ey};
                 r = tile_rect(e, v);
                 cand = rect_candidates(r);
             }
         }
-        uint32_t mask;
+        if (!sh_asked) {
+            // the barrier also publishes s_bar
+            sh_asked = __syncthreads_or(cand > 0) != 0;
+            if (sh_asked && threadIdx.x == 0) ask_sh();
+        }
+        if (a.probe_xy && valid) {
+            const int64_t q = (int64_t)view * a.n + gid;
+            a.probe_xy[q] = projected ? make_float2(s.x, s.y) : make_float2(-128.0f, -128.0f);
+            a.probe_z[q] = projected ? s.z : -128.0f;
+            a.probe_ell[q] = projected ? make_float4(s.cs, s.sn, s.ex, s.ey) : make_float4(0.f, 0.f, 0.f, 0.f);
+            a.probe_conic[q] = projected ? make_float4(s.ca, s.cb, s.cc, 0.0f) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
         // the overlap test is the reference's in every mode: the tile lists
         // of the projected floats are exactly those of the reference's build
-        const int hits = warp_count_hits(e, r, cand, v, mask, BUCKET ? a.tile_count : nullptr, a.aggregate != 0);
-        int64_t o_out = o;  // where this item's outputs go
-        if (BUCKET) {
-            const unsigned bal = __ballot_sync(kFull, hits > 0);
-            if (bal == 0) continue;  // warp-uniform
-            unsigned long long first = 0;
-            if ((threadIdx.x & 31) == 0) first = atomicAdd(a.slot_counter, (unsigned long long)__popc(bal));
-            first = __shfl_sync(kFull, first, 0);
-            o_out = (int64_t)first + __popc(bal & lanemask_lt());
-            if (hits > 0) a.offsets[o_out] = (int32_t)((int64_t)view * a.n + gid);
-        } else {
-            const int64_t off = chain_offsets(hits, a.status + (int64_t)view * a.groups, group, a.groups, epoch,
-                                              a.view_total + view, a.err);
-            if (valid) a.offsets[o] = (int32_t)off;
-        }
-        if (valid) {
-            const int64_t o = o_out;
-            if (a.probe_xy) {
-                const int64_t q = (int64_t)view * a.n + gid;
-                if (projected) {
-                    a.probe_xy[q] = make_float2(s.x, s.y);
-                    a.probe_z[q] = s.z;
-                    a.probe_ell[q] = make_float4(s.cs, s.sn, s.ex, s.ey);
-                    a.probe_conic[q] = make_float4(s.ca, s.cb, s.cc, 0.0f);
+        if constexpr (BUCKET) {
+            const unsigned owners = __ballot_sync(kFull, cand > 0);
+            if (owners == 0) continue;  // warp-uniform
+            const bool large = cand > kLargeCandidates;
+            OverlapPending x;
+            const BucketWalk k = start_walk(e, r, large ? 0 : cand, v, a, owners, x);
+            const int2 pr = pack_rect(r);
+            // what the walk has no registers for
+            if (cand > 0) s_geom[threadIdx.x] = make_float4(s.ca, s.cb, s.cc, s.z);
+            unsigned mine;
+            const unsigned reached = run_walk(e, pr, v, a, k, a.probe_color != nullptr, x, mine);
+            const unsigned long long got = __shfl_sync(kFull, k.got, 0);
+            const uint32_t o = (uint32_t)got + (uint32_t)__popc(owners & lanemask_lt());
+            if (cand > 0) {
+                const float4 g = s_geom[threadIdx.x];
+                a.offsets[o] = view * (int32_t)a.n + gid;
+                a.depth[o] = depth_bits(g.w);
+                if (large) {
+                    a.rect[o] = pr;
+                    a.ell[o] = make_float4(e.cs, e.sn, e.ex, e.ey);
+                }
+                if (a.raster_mode == 0 || large) a.xy[o] = make_float2(e.cx, e.cy);
+                // the colour only matters for items that can reach a tile
+                const float4 col = colour(v);
+                if (a.raster_mode == 0) {
+                    a.conic[o] = make_float4(g.x, g.y, g.z, 0.0f);
+                    a.color[o] = col;
                 } else {
-                    a.probe_xy[q] = make_float2(-128.0f, -128.0f);
-                    a.probe_z[q] = -128.0f;
-                    a.probe_ell[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    a.probe_conic[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    write_record(a.rec + 3 * (int64_t)o, e, g, col);
+                }
+                if (a.probe_color) {
+                    // a large splat reaches a tile unless an extent is zero
+                    // (ellipse_rect_overlap_clear) and its centre is on a border
+                    int t0;
+                    const bool hit = large ? (e.ex != 0.0f && e.ey != 0.0f) ||
+                                                 centre_candidate(e, unpack_rect(pr), cand, v, t0) >= 0
+                                           : ((reached >> (threadIdx.x & 31)) & 1u) != 0;
+                    if (hit) a.probe_color[(int64_t)view * a.n + gid] = col;
                 }
             }
+            const int lane = threadIdx.x & 31, steps = (k.total + 31) >> 5;
+            const uint32_t chunk = (uint32_t)(got >> 32) + (k.preb ? 1u : 0u);  // of step 0
+            write_pending(a, x, chunk + (uint32_t)steps - 1u);
+            if (lane < steps && chunk + (uint32_t)lane < a.chunk_capacity)
+                a.chunks[chunk + (uint32_t)lane] = make_uint4(mine, (uint32_t)got, owners, 0u);
+            if (lane == 0 && k.preb && chunk - 1u < a.chunk_capacity)
+                a.chunks[chunk - 1u] = make_uint4(k.preb, (uint32_t)got, owners, 0u);
+            if (__any_sync(kFull, large)) list_large(cand, large, o, a);
+        } else {
+            uint32_t mask;
+            const int hits = warp_count_hits(e, r, cand, v, mask);
+            const int64_t off = chain_offsets(hits, a.status + (int64_t)view * a.groups, group, a.groups, epoch,
+                                              a.view_total + view, a.err);
+            const int64_t o = (int64_t)view * a.n + i;
+            if (valid) a.offsets[o] = (int32_t)off;
             if (hits > 0) {
-                // the colour only matters for items that reach a tile, so the
-                // SH evaluation runs after the overlap test
-                if (DEG >= 0) {
-                    const float3 d = view_dir(v, p);
-                    const float3 c = sh_color<DEG, false>(d.x, d.y, d.z, s_sh + threadIdx.x, 256);
-                    col = make_float4(c.x, c.y, c.z, p.w);
-                }
-                if (a.probe_color) a.probe_color[(int64_t)view * a.n + gid] = col;
+                const float4 col = colour(v);
                 a.z[o] = s.z;
                 a.rect[o] = pack_rect(r);
                 a.hitmask[o] = mask;
@@ -413,30 +707,13 @@ __global__ void __launch_bounds__(256, (DEG >= 3 && !FAST) ? 3 : 4) frame_projec
                     a.color[o] = col;
                     a.conic[o] = make_float4(s.ca, s.cb, s.cc, 0.0f);
                 } else {
-                    float ex, ey, A = -0.72134752f * s.ca, B = -1.44269504f * s.cb, C = -0.72134752f * s.cc;
-                    float L = lg2_approx(col.w);
-                    const float det = s.ca * s.cc - s.cb * s.cb;
-                    if (!(det > 0.0f) || !(s.ca > 0.0f) || !(s.cc > 0.0f) || !(col.w > kCullAlpha)) {
-                        // contributes nothing anywhere: alpha below the cutoff,
-                        // or a conic that is not positive definite
-                        ex = ey = -1e30f;
-                        A = B = C = 0.0f;
-                        L = -1e30f;
-                    } else {
-                        // qc = 2 ln(opacity / cutoff) = 2 ln 2 (L + 18); 1.0001
-                        // covers the approximations
-                        const float qc = 1.38643f * (L + 18.0f);
-                        const float rdet = rcp_approx(det);
-                        ex = sqrt_approx(qc * s.cc * rdet);
-                        ey = sqrt_approx(qc * s.ca * rdet);
-                    }
-                    a.rec[3 * o + 0] = make_float4(s.x, s.y, ex, ey);
-                    a.rec[3 * o + 1] = make_float4(A, B, C, L);
-                    a.rec[3 * o + 2] = make_float4(col.x, col.y, col.z, 0.0f);
+                    write_record(a.rec + 3 * o, e, make_float4(s.ca, s.cb, s.cc, s.z), col);
                 }
             }
         }
     }
+    // the copy lands before the block's shared memory goes to another one
+    if (DEG >= 0 && threadIdx.x == 0 && sh_asked && !sh_here) sh_wait(&s_bar, a.err);
 }
 
 // Count-only variant for the stage API: rectangle + exact count + scan from
@@ -608,17 +885,26 @@ void launch_project_stage(int64_t n, const float4* pos, const float4* sr, const 
     project_stage_kernel<<<grid, 256, 0, st>>>(n, pos, sr, v, xy, z, ell, conic);
 }
 
-template <int DEG, bool BUCKET, bool FAST>
-static void launch_frame_deg(const FrameArgs& a, cudaStream_t st)
+template <int DEG, bool BUCKET, bool FAST, bool MANY>
+static void launch_frame_views(const FrameArgs& a, cudaStream_t st)
 {
     constexpr int NCOEF = DEG >= 0 ? 3 * (DEG + 1) * (DEG + 1) : 0;
     constexpr int smem = NCOEF * 256 * (int)sizeof(float);
     static PerDeviceOnce attr;
     attr.run([] {
-        cudaFuncSetAttribute(frame_project_kernel<DEG, BUCKET, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem);
+        cudaFuncSetAttribute(frame_project_kernel<DEG, BUCKET, FAST, MANY>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     });
-    frame_project_kernel<DEG, BUCKET, FAST><<<(unsigned)a.num_tiles, 256, smem, st>>>(a);
+    frame_project_kernel<DEG, BUCKET, FAST, MANY><<<(unsigned)a.num_tiles, 256, smem, st>>>(a);
+}
+
+template <int DEG, bool BUCKET, bool FAST>
+static void launch_frame_deg(const FrameArgs& a, cudaStream_t st)
+{
+    if (a.views_per_block > 1)
+        launch_frame_views<DEG, BUCKET, FAST, true>(a, st);
+    else
+        launch_frame_views<DEG, BUCKET, FAST, false>(a, st);
 }
 
 template <bool BUCKET, bool FAST>
@@ -647,6 +933,11 @@ void launch_frame_project(const FrameArgs& a, int deg, cudaStream_t st, bool buc
         launch_frame_mode<false, true>(a, deg, st);
     else
         launch_frame_mode<false, false>(a, deg, st);
+}
+
+void launch_large_overlaps(const FrameArgs& a, int num_sms, cudaStream_t st)
+{
+    large_overlap_kernel<<<(unsigned)(num_sms * 4), 256, 0, st>>>(a);
 }
 
 void launch_count_stage(const FrameArgs& a, cudaStream_t st)
