@@ -105,9 +105,10 @@ struct DevBuf {
     }
 };
 
-// Small per-context device words, reset at the start of every frame (by a
-// copy of the pinned `h_init`, which also carries the frame's look-back
-// epochs, so a captured frame reads fresh epochs on every replay).
+// Small device words, reset at the start of every frame.  A bucket frame's are
+// copied from the pinned `h_init`, which also carries the frame's look-back
+// epochs, so a captured frame reads fresh epochs on every replay; the view
+// parameters follow at kViewsOffset, so that one copy brings both.
 struct Counters {
     unsigned long long frame_tile;                 // frame kernel block queue
     unsigned long long raster_tile;                // persistent raster queue
@@ -122,12 +123,12 @@ struct Counters {
     int64_t sort_n;                                // min(K, key capacity)
     unsigned int big_tiles;                        // tiles sorted ahead of the raster (to 4096 keys)
     unsigned int huge_tiles;                       // those above 4096 keys
-    unsigned int class_tiles[kOrderClasses];       // raster order: tiles of each class, and
-    unsigned int class_heads[kOrderClasses];       // how many of them are placed
     int err;
     int overflow;                                  // the key or overlap list was too short: redo the frame
     uint32_t epoch_scan, epoch_sort;               // look-back epochs of this frame
 };
+
+constexpr size_t kViewsOffset = (sizeof(Counters) + 255) & ~(size_t)255;
 
 // A frame captured into a CUDA graph, or a frame seen once (no `exec` yet):
 // the graph is captured the second time the same key comes along.
@@ -141,26 +142,55 @@ struct FrameGraph {
     uint64_t last_use = 0;
     int seen = 0;                    // calls with this key
     int failed = 0;                  // capture failed: run this key without a graph
-    int raster_groups = 0;           // raster launched per view group (host-output batches)
+    int raster_groups = 0;           // raster launched in groups (host-output frames)
     int split = 0;                   // needed 2^31 tile keys or more: render as halves of the views
 };
 constexpr size_t kMaxGraphs = 8;
-// gs_render_batch_host renders batches of more than this many views in
-// groups, reading each group back while the next one renders.
+// gs_render_batch_host renders reference-mode and onesweep batches in frames of
+// this many views.
 constexpr int kHostChunkViews = 16;
-constexpr int kHostGroupViews = 8;  // views per raster group of a T_min host batch
-constexpr int kMaxRasterGroups = 8;
+// Image bytes per raster group of a host-output frame: a copy of this size
+// takes 36 us at 55 GB/s, several times its launch and its group's.
+constexpr size_t kHostGroupBytes = 2u << 20;
 
-// Host read-back overlapped with the frame (T_min bucket frames): the
-// raster runs one view group after the other, each group's end is marked by
-// an event, and the group's images are copied on `copy` after it.
+// Host read-back overlapped with the frame (bucket frames): the raster runs in
+// groups of tile rows, one after the other in image order, each group's end is
+// marked by an event, and its part of the images is copied on `copy` after it.
 struct HostCopy {
     uint8_t* h_rgba = nullptr;
+    const uint8_t* d_rgba = nullptr;  // all views' images, one after the other
     cudaStream_t copy = nullptr;
     int groups = 0;
-    int first_view[kMaxRasterGroups + 1] = {};  // group g = views [first_view[g], first_view[g + 1])
+    int64_t first_tile[kMaxRasterGroups + 1] = {};  // group g = global tiles [first_tile[g], first_tile[g + 1])
     size_t first_byte[kMaxRasterGroups + 1] = {};
 };
+
+// Cuts the views' tile rows into groups of about equal size; the last one,
+// whose copy nothing overlaps, is a quarter of the others.
+void plan_host_copy(const gs_camera* cams, int num_views, const gs_render_cfg& cfg, HostCopy& hc)
+{
+    size_t total = 0;
+    for (int v = 0; v < num_views; ++v) total += 4 * (size_t)cams[v].width * cams[v].height;
+    const int want = (int)std::min<size_t>(kMaxRasterGroups, std::max<size_t>(1, total / kHostGroupBytes));
+    const double share = (double)total / (want > 1 ? want - 0.75 : 1.0);
+    int64_t tile = 0;
+    size_t byte = 0;
+    hc.groups = 0;
+    for (int v = 0; v < num_views; ++v) {
+        const int64_t tx = (cams[v].width + cfg.tile_w - 1) / cfg.tile_w, ty = (cams[v].height + cfg.tile_h - 1) / cfg.tile_h;
+        for (int64_t row = 0; row < ty; ++row) {
+            // group g starts with the first row at or past g shares
+            if (hc.groups == 0 || (hc.groups < want && (double)byte >= hc.groups * share)) {
+                hc.first_tile[hc.groups] = tile;
+                hc.first_byte[hc.groups++] = byte;
+            }
+            tile += tx;
+            byte += 4 * (size_t)cams[v].width * (size_t)std::min<int64_t>(cfg.tile_h, cams[v].height - row * cfg.tile_h);
+        }
+    }
+    hc.first_tile[hc.groups] = tile;
+    hc.first_byte[hc.groups] = byte;
+}
 
 // A tuned bucket of gs_autotune: the batching knobs that were fastest for
 // scenes of 2^n_log2 .. 2^(n_log2+1) Gaussians, views of 2^px_log2 ..
@@ -212,7 +242,7 @@ struct gs_ctx {
     int num_sms = 148;
     std::mutex mu;
     uint32_t epoch_scan = 1, epoch_sort = 1;
-    DevBuf views;                          // ViewParams[]
+    DevBuf views;                          // Counters of a bucket frame, then at kViewsOffset ViewParams[]
     DevBuf color, xy, z, ell, conic, rect, offsets;  // per (view, Gaussian)
     DevBuf rec, hitmask;                   // T_min raster records (48 B), candidate hit masks
     DevBuf scan_status;                    // frame kernel look-back words, [view][group]
@@ -224,17 +254,21 @@ struct gs_ctx {
     DevBuf overlaps, chunks;               // tile-bucket ordering: the frame's overlap list (BucketEmitArgs)
     int64_t chunk_capacity = 0;
     DevBuf tile_order;                     // raster order of the tiles (heavy tiles first)
-    DevBuf counters;
+    DevBuf counters;                       // of the other paths
+    DevBuf classes;                        // raster order: tiles of each class, and how many of them are placed
     DevBuf image;                          // images of the host-output variants
-    Counters* h_counters = nullptr;        // pinned mirror
-    Counters* h_init = nullptr;            // pinned per-frame reset image of the counters
-    ViewParams* h_views = nullptr;         // pinned staging
+    Counters* h_counters = nullptr;        // pinned mirror of `counters`
+    FrameResult* h_result = nullptr;       // pinned; written by the emission of a bucket frame
+    Counters* h_init = nullptr;            // pinned image of `views`: the reset counters, then
+    ViewParams* h_views = nullptr;         // the view parameters at kViewsOffset
     int h_views_cap = 0;
     cudaEvent_t ev[8] = {};
     int64_t key_capacity = 0;
     cudaStream_t cap_stream = nullptr;     // graph capture
     cudaStream_t copy_stream = nullptr;    // image read-back of the host-output batches
-    cudaEvent_t ev_group[kMaxRasterGroups] = {};  // end of each raster view group
+    cudaStream_t raster_stream = nullptr;  // every other raster group of a host-output frame
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_group[kMaxRasterGroups] = {};  // end of each raster group
     bool tile_count_dirty = true;          // tile counts may be nonzero: clear before the next frame
     std::vector<FrameGraph> graphs;
     uint64_t use_clock = 0;
@@ -346,15 +380,22 @@ uint32_t take_epochs(uint32_t& epoch, uint32_t count, DevBuf& status, cudaStream
     return e;
 }
 
+ViewParams* views_of(const gs_ctx* ctx) { return reinterpret_cast<ViewParams*>(ctx->views.as<char>() + kViewsOffset); }
+
 int ensure_ctx_host(gs_ctx* ctx, int num_views)
 {
+    const size_t bytes = kViewsOffset + sizeof(ViewParams) * (size_t)num_views;
     if (num_views > ctx->h_views_cap) {
-        if (ctx->h_views) cudaFreeHost(ctx->h_views);
+        if (ctx->h_init) cudaFreeHost(ctx->h_init);
+        ctx->h_init = nullptr;
         ctx->h_views = nullptr;
-        GS_CUDA(cudaMallocHost(&ctx->h_views, sizeof(ViewParams) * (size_t)num_views));
+        ctx->h_views_cap = 0;
+        GS_CUDA(cudaMallocHost(&ctx->h_init, bytes));
+        std::memset(ctx->h_init, 0, kViewsOffset);
+        ctx->h_views = reinterpret_cast<ViewParams*>(reinterpret_cast<char*>(ctx->h_init) + kViewsOffset);
         ctx->h_views_cap = num_views;
     }
-    if (ctx->views.ensure(sizeof(ViewParams) * (size_t)num_views) != cudaSuccess) return fail(GS_ERR_OOM, "views");
+    if (ctx->views.ensure(bytes) != cudaSuccess) return fail(GS_ERR_OOM, "views");
     return GS_OK;
 }
 
@@ -447,7 +488,7 @@ int run_frame_onesweep(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams
     if (ctx->ranges.ensure(sizeof(int32_t) * 2 * (size_t)tiles_total)) return fail(GS_ERR_OOM, "ranges");
 
     Counters* dc = ctx->counters.as<Counters>();
-    GS_CUDA(cudaMemcpyAsync(ctx->views.p, ctx->h_views, sizeof(ViewParams) * num_views, cudaMemcpyHostToDevice, st));
+    GS_CUDA(cudaMemcpyAsync(views_of(ctx), ctx->h_views, sizeof(ViewParams) * num_views, cudaMemcpyHostToDevice, st));
     GS_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), st));
     GS_CUDA(cudaEventRecord(ctx->ev[0], st));
 
@@ -465,7 +506,7 @@ int run_frame_onesweep(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams
     fa.sh = scene->sh.as<float>();
     fa.sh_count = scene->sh_count;
     fa.color_in = scene->color.as<float4>();
-    fa.views = ctx->views.as<ViewParams>();
+    fa.views = views_of(ctx);
     fa.color = ctx->color.as<float4>();
     fa.xy = ctx->xy.as<float2>();
     fa.z = ctx->z.as<float>();
@@ -508,7 +549,7 @@ int run_frame_onesweep(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams
     EmitArgs ea{};
     ea.n = n;
     ea.num_views = num_views;
-    ea.views = ctx->views.as<ViewParams>();
+    ea.views = views_of(ctx);
     ea.offsets = ctx->offsets.as<int32_t>();
     ea.view_total = view_total;
     ea.view_base = view_base;
@@ -549,7 +590,7 @@ int run_frame_onesweep(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams
     if (K > 0) launch_ranges(skeys, K, nullptr, ctx->ranges.as<int32_t>(), st);
     RasterArgs ra{};
     ra.view0 = ctx->h_views[0];
-    ra.views = ctx->views.as<ViewParams>();
+    ra.views = views_of(ctx);
     ra.num_views = num_views;
     ra.write_empty = 1;
     ra.num_tiles_total = tiles_total;
@@ -593,7 +634,7 @@ struct FramePlan {
     int num_views = 0;
     int64_t n = 0, groups = 0, blocks = 0, items = 0, tiles_total = 0;
     int vpb = 0, deg = 0;
-    const HostCopy* host_copy = nullptr;  // non-null: raster per view group, each group's end marked
+    const HostCopy* host_copy = nullptr;  // non-null: raster in groups, each group's end marked
     const gs_frame_probe* probe = nullptr;  // non-null: the frame kernel also writes the probe outputs
 };
 
@@ -653,15 +694,13 @@ int plan_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams,
 
 // Enqueues a whole tile-bucket frame on `st` with no host synchronisation
 // (everything a replayed graph needs): counters reset, fused projection,
-// tile scan, bucket emit, tile sort, raster, counters read-back into
-// ctx->h_counters.  The key count stays on the device; a frame whose keys
+// tile scan, bucket emit (which reports to ctx->h_result), tile sort, raster.  The key count stays on the device; a frame whose keys
 // exceed ctx->key_capacity comes back with `overflow` set.
 int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg& cfg, const FramePlan& p,
                          cudaStream_t st, bool capturing)
 {
-    Counters* dc = ctx->counters.as<Counters>();
-    GS_CUDA(cudaMemcpyAsync(ctx->views.p, ctx->h_views, sizeof(ViewParams) * p.num_views, cudaMemcpyHostToDevice, st));
-    GS_CUDA(cudaMemcpyAsync(dc, ctx->h_init, sizeof(Counters), cudaMemcpyHostToDevice, st));
+    Counters* dc = ctx->views.as<Counters>();
+    GS_CUDA(cudaMemcpyAsync(dc, ctx->h_init, kViewsOffset + sizeof(ViewParams) * p.num_views, cudaMemcpyHostToDevice, st));
     // the tile counts are all zero here: cleared when allocated, re-zeroed
     // by every tile scan, and cleared again after a failed frame
     if (ctx->tile_count_dirty) {
@@ -682,7 +721,7 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     fa.sh = scene->sh.as<float>();
     fa.sh_count = scene->sh_count;
     fa.color_in = scene->color.as<float4>();
-    fa.views = ctx->views.as<ViewParams>();
+    fa.views = views_of(ctx);
     fa.raster_mode = cfg.termination;
     fa.color = ctx->color.as<float4>();
     fa.xy = ctx->xy.as<float2>();
@@ -710,6 +749,8 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
         fa.probe_conic = reinterpret_cast<float4*>(p.probe->d_conic);
         fa.probe_color = reinterpret_cast<float4*>(p.probe->d_color);
     }
+    fa.zero_words = ctx->classes.as<unsigned int>();
+    fa.zero_count = 2 * kMaxRasterGroups * kOrderClasses;
     if (p.n > 0) {
         launch_frame_project(fa, p.deg, st, true);
         launch_large_overlaps(fa, ctx->num_sms, st);
@@ -735,10 +776,12 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ta.big_count = &dc->big_tiles;
     ta.huge_count = &dc->huge_tiles;
     ta.fused_cap = fused_tile_capacity(cfg.tile_w, cfg.tile_h);
-    ta.class_tiles = dc->class_tiles;
+    ta.class_tiles = ctx->classes.as<unsigned int>();
+    const bool in_groups = p.host_copy && p.host_copy->groups > 1;
+    ta.groups = in_groups ? p.host_copy->groups : 1;
+    for (int g = 0; g < ta.groups; ++g) ta.group_tile[g] = in_groups ? p.host_copy->first_tile[g] : 0;
     launch_tile_scan(ta, st);
     GS_CUDA(record(ctx->ev[1], st, capturing));
-    GS_CUDA(record(ctx->ev[2], st, capturing));
 
     BucketEmitArgs ea{};
     ea.slot_counter = &dc->slots;
@@ -752,14 +795,17 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ea.err = &dc->err;
     ea.big_count = &dc->big_tiles;
     ea.huge_count = &dc->huge_tiles;
-    const bool in_groups = p.host_copy && p.host_copy->groups > 1 && cfg.termination == GS_TERM_TMIN;
-    const bool in_order = !in_groups && p.n > 0;
-    ea.order = in_order ? ctx->tile_order.as<int32_t>() : nullptr;
-    ea.class_tiles = dc->class_tiles;
-    ea.class_heads = dc->class_heads;
+    ea.order = p.n > 0 ? ctx->tile_order.as<int32_t>() : nullptr;
+    ea.total = &dc->total;
+    ea.unit_count = &dc->units;
+    ea.result = ctx->h_result;
+    ea.groups = ta.groups;
+    std::copy(ta.group_tile, ta.group_tile + kMaxRasterGroups, ea.group_tile);
+    ea.class_tiles = ta.class_tiles;
+    ea.class_heads = ta.class_tiles + kMaxRasterGroups * kOrderClasses;
     ea.keys = ctx->keys0.as<uint64_t>();
     ea.batch_counter = &dc->emit_batch;
-    if (p.n > 0) launch_emit_bucket(ea, ctx->num_sms, st);
+    launch_emit_bucket(ea, ctx->num_sms, st);
     GS_CUDA(record(ctx->ev[3], st, capturing));
 
     TileSortArgs sa{};
@@ -779,7 +825,7 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
 
     RasterArgs ra{};
     ra.view0 = ctx->h_views[0];
-    ra.views = ctx->views.as<ViewParams>();
+    ra.views = views_of(ctx);
     ra.num_views = p.num_views;
     ra.write_empty = 1;
     ra.num_tiles_total = p.tiles_total;
@@ -799,27 +845,35 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ra.rec_persistent = cfg.raster_persistent;
     ra.sort_prefix_bits = cfg.sort_bits;
     if (in_groups) {
-        // one launch per view group, in view order; a group's images are
-        // complete at its event
+        // one launch per group, in image order; a group's rows are complete at
+        // its event.  The groups alternate between two streams, so that one's
+        // last CTAs run beside the next one's first (not the persistent
+        // raster's: its groups share the tile queue).
         const HostCopy& hc = *p.host_copy;
+        const bool fork = !ra.rec_persistent;
+        if (fork) {
+            GS_CUDA(cudaEventRecord(ctx->ev_fork, st));
+            GS_CUDA(cudaStreamWaitEvent(ctx->raster_stream, ctx->ev_fork, 0));
+        }
         for (int g = 0; g < hc.groups; ++g) {
-            const int v0 = hc.first_view[g], v1 = hc.first_view[g + 1];
-            const int64_t t0 = ctx->h_views[v0].tile_offset;
-            const int64_t t1 = v1 < p.num_views ? ctx->h_views[v1].tile_offset : p.tiles_total;
+            cudaStream_t gst = fork && (g & 1) ? ctx->raster_stream : st;
             RasterArgs rg = ra;
-            rg.tile_base = t0;
-            rg.num_tiles_total = t1 - t0;
+            rg.tile_base = hc.first_tile[g];
+            rg.num_tiles_total = hc.first_tile[g + 1] - hc.first_tile[g];
             // a persistent group launch starts its own queue from zero
-            if (rg.rec_persistent) GS_CUDA(cudaMemsetAsync(&dc->raster_tile, 0, sizeof(unsigned long long), st));
-            launch_raster(rg, cfg.tile_w, cfg.tile_h, cfg.termination, ctx->num_sms, st);
-            GS_CUDA(record(ctx->ev_group[g], st, capturing));
+            if (rg.rec_persistent) GS_CUDA(cudaMemsetAsync(&dc->raster_tile, 0, sizeof(unsigned long long), gst));
+            launch_raster(rg, cfg.tile_w, cfg.tile_h, cfg.termination, ctx->num_sms, gst);
+            GS_CUDA(record(ctx->ev_group[g], gst, capturing));
+        }
+        if (fork) {
+            GS_CUDA(cudaEventRecord(ctx->ev_join, ctx->raster_stream));
+            GS_CUDA(cudaStreamWaitEvent(st, ctx->ev_join, 0));
         }
     } else {
         launch_raster(ra, cfg.tile_w, cfg.tile_h, cfg.termination, ctx->num_sms, st);
     }
     GS_CUDA(cudaGetLastError());
     GS_CUDA(record(ctx->ev[5], st, capturing));
-    GS_CUDA(cudaMemcpyAsync(ctx->h_counters, dc, sizeof(Counters), cudaMemcpyDeviceToHost, st));
     return GS_OK;
 }
 
@@ -829,7 +883,7 @@ uint64_t layout_of(const gs_ctx* ctx)
     const DevBuf* bufs[] = {&ctx->views, &ctx->color, &ctx->xy, &ctx->z, &ctx->ell, &ctx->conic, &ctx->rect,
                             &ctx->offsets, &ctx->rec, &ctx->hitmask, &ctx->scan_status, &ctx->keys0, &ctx->vals0,
                             &ctx->keys1, &ctx->vals1, &ctx->ranges, &ctx->tile_count, &ctx->big_list,
-                            &ctx->tile_order, &ctx->counters, &ctx->overlaps, &ctx->chunks};
+                            &ctx->tile_order, &ctx->classes, &ctx->overlaps, &ctx->chunks};
     uint64_t h = 1469598103934665603ull;
     auto mix = [&h](uint64_t x) { h = (h ^ x) * 1099511628211ull; };
     for (const DevBuf* b : bufs) {
@@ -955,14 +1009,13 @@ int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, 
             if (rc) return rc;
             replayed = false;
         }
-        if (hc && hc->groups > 1 && cfg.termination == GS_TERM_TMIN) {
-            // each group's images go to the host once its raster is done,
-            // while the next group renders (a redone frame copies again)
+        if (hc && hc->groups > 1) {
+            // each group's rows go to the host once its raster is done, while
+            // the next group renders (a redone frame copies again)
             for (int gi = 0; gi < hc->groups; ++gi) {
                 GS_CUDA(cudaStreamWaitEvent(hc->copy, ctx->ev_group[gi], 0));
                 const size_t b0 = hc->first_byte[gi], b1 = hc->first_byte[gi + 1];
-                GS_CUDA(cudaMemcpyAsync(hc->h_rgba + b0, outs[hc->first_view[gi]], b1 - b0, cudaMemcpyDeviceToHost,
-                                        hc->copy));
+                GS_CUDA(cudaMemcpyAsync(hc->h_rgba + b0, hc->d_rgba + b0, b1 - b0, cudaMemcpyDeviceToHost, hc->copy));
             }
         }
         const cudaError_t se = cudaStreamSynchronize(st);
@@ -970,45 +1023,44 @@ int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, 
             ctx->tile_count_dirty = true;
             return cuda_fail(se, "frame");
         }
-        if (ctx->h_counters->err) {
+        if (ctx->h_result->err) {
             ctx->tile_count_dirty = true;
             return fail(GS_ERR_DEVICE_TIMEOUT, "frame look-back timed out");
         }
-        const int64_t K = ctx->h_counters->total;
+        const int64_t K = ctx->h_result->total;
         if (K >= (1ll << 31)) {
             if (g) g->split = 1;
             return fail(kSplitViews, "more than 2^31 tile keys");
         }
-        if (!ctx->h_counters->overflow) break;
+        if (!ctx->h_result->overflow) break;
         if (attempts >= 3) return fail(GS_ERR_CUDA, "tile list overflow after regrowing");
         if (g) drop_graph(*g);
         // (the key and chunk counts are exact unless large splats' units did not fit)
-        const int64_t need = std::max(K > ctx->key_capacity ? K + K / 4 : 0, (int64_t)ctx->h_counters->units);
+        const int64_t need = std::max(K > ctx->key_capacity ? K + K / 4 : 0, (int64_t)ctx->h_result->units);
         rc = ensure_key_buffers(ctx, std::min<int64_t>(need, (1ll << 31) - 1));
         if (rc) return rc;
-        const int64_t chunks = (int64_t)(ctx->h_counters->slots >> 32);
+        const int64_t chunks = (int64_t)(ctx->h_result->slots >> 32);
         rc = ensure_overlaps(ctx, chunks);
         if (rc) return rc;
     }
 
     ctx->last_tiles = p.tiles_total;
-    ctx->last_keys = ctx->h_counters->total;
-    ctx->last_slots = (int64_t)(ctx->h_counters->slots & 0xFFFFFFFFull);
+    ctx->last_keys = ctx->h_result->total;
+    ctx->last_slots = (int64_t)(ctx->h_result->slots & 0xFFFFFFFFull);
     ctx->last_fused_cap = fused_tile_capacity(cfg.tile_w, cfg.tile_h);
     if (stats) {
         stats->sh_eval_ms = 0.0;
         stats->project_ms = ms_between(ctx->ev[0], ctx->ev[1]);
-        stats->build_tile_ms = ms_between(ctx->ev[2], ctx->ev[3]);
+        stats->build_tile_ms = ms_between(ctx->ev[1], ctx->ev[3]);
         stats->sort_ms = ms_between(ctx->ev[3], ctx->ev[4]);  // the tiles too big for the raster CTAs
         stats->raster_ms = ms_between(ctx->ev[4], ctx->ev[5]);
         stats->total_ms = ms_between(ctx->ev[0], ctx->ev[5]);
-        stats->num_keys = ctx->h_counters->total;
+        stats->num_keys = ctx->h_result->total;
         stats->num_tiles = p.tiles_total;
-        // frame kernel, large splats, bucket emit, the two big-tile sorts; tile scan,
-        // raster (sorts the other tiles; one launch per view group when the
-        // images stream to host memory group by group)
-        const bool grouped = p.host_copy && p.host_copy->groups > 1 && cfg.termination == GS_TERM_TMIN;
-        stats->kernel_launches = (p.n > 0 ? 5 : 0) + 1 + (grouped ? p.host_copy->groups : 1);
+        // frame kernel, large splats, the two big-tile sorts; tile scan, bucket emit,
+        // raster (sorts the other tiles; one launch per group when the images
+        // stream to host memory)
+        stats->kernel_launches = (p.n > 0 ? 4 : 0) + 2 + std::max(1, raster_groups);
         stats->graph_replay = replayed ? 1 : 0;
         stats->attempts = attempts;
     }
@@ -1063,6 +1115,54 @@ int run_frame(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, int num
     if (rc != kSplitViews) return rc;
     if (num_views == 1) return fail(GS_ERR_CAPACITY, "more than 2^31 tile keys in one view");
     return run_frame_halves(ctx, scene, cams, num_views, cfg, outs, stats, st, 1);
+}
+
+// One bucket frame whose images (one after the other at outs[0]) stream to host
+// memory while it renders, as plan_host_copy groups them.  Returns when every
+// image is there.
+int run_grouped_frame(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, int num_views,
+                      const gs_render_cfg& cfg, uint8_t* const* outs, uint8_t* h_rgba, gs_stats* stats, cudaStream_t st)
+{
+    if (!valid_cfg(cfg)) return fail(GS_ERR_INVALID, "invalid render cfg");
+    if (!ctx->copy_stream) GS_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
+    if (!ctx->raster_stream) GS_CUDA(cudaStreamCreateWithFlags(&ctx->raster_stream, cudaStreamNonBlocking));
+    if (!ctx->ev_fork) GS_CUDA(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
+    if (!ctx->ev_join) GS_CUDA(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
+    HostCopy hc;
+    plan_host_copy(cams, num_views, cfg, hc);
+    hc.h_rgba = h_rgba;
+    hc.d_rgba = outs[0];
+    hc.copy = ctx->copy_stream;
+    const int rc = run_frame_bucket(ctx, scene, cams, num_views, cfg, outs, stats, st, &hc);
+    cudaError_t se = hc.groups > 1 ? cudaStreamSynchronize(ctx->copy_stream) : cudaSuccess;
+    if (rc) return rc;
+    if (hc.groups == 1) {
+        se = cudaMemcpyAsync(h_rgba, outs[0], hc.first_byte[1], cudaMemcpyDeviceToHost, st);
+        if (se == cudaSuccess) se = cudaStreamSynchronize(st);
+    }
+    return se == cudaSuccess ? GS_OK : cuda_fail(se, "image copy");
+}
+
+// One frame into host memory, in any ordering: bucket frames stream their
+// images, the others copy them once they are done.
+int run_host_frame(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, int num_views, const gs_render_cfg& cfg_in,
+                   uint8_t* const* outs, size_t bytes, uint8_t* h_rgba, gs_stats* stats, cudaStream_t st)
+{
+    gs_render_cfg cfg = cfg_in;
+    if (cfg.ordering == GS_ORDER_AUTO) cfg.ordering = GS_ORDER_BUCKETS;  // not tuned: the default ordering
+    int rc = kSplitViews, tried = 0;
+    if (cfg.ordering == GS_ORDER_BUCKETS && scene->n * (int64_t)num_views < (1ll << 31)) {
+        rc = run_grouped_frame(ctx, scene, cams, num_views, cfg, outs, h_rgba, stats, st);
+        if (rc != kSplitViews) return rc;
+        if (num_views == 1) return fail(GS_ERR_CAPACITY, "more than 2^31 tile keys in one view");
+        tried = 1;
+    }
+    rc = tried ? run_frame_halves(ctx, scene, cams, num_views, cfg, outs, stats, st, tried)
+               : run_frame(ctx, scene, cams, num_views, cfg, outs, stats, st);
+    if (rc) return rc;
+    GS_CUDA(cudaMemcpyAsync(h_rgba, outs[0], bytes, cudaMemcpyDeviceToHost, st));
+    GS_CUDA(cudaStreamSynchronize(st));
+    return GS_OK;
 }
 
 // floor(log2(x)) for x >= 1, -1 for x <= 0
@@ -1247,18 +1347,21 @@ int gs_ctx_create(int device, gs_ctx** out)
     if (!c) return fail(GS_ERR_OOM, "host allocation");
     c->device = device;
     c->num_sms = prop.multiProcessorCount;
-    if (c->counters.ensure(sizeof(Counters), true) != cudaSuccess) {
+    if (c->counters.ensure(sizeof(Counters), true) != cudaSuccess ||
+        c->classes.ensure(sizeof(unsigned int) * 2 * kMaxRasterGroups * kOrderClasses, true) != cudaSuccess) {
+        c->counters.release();
         delete c;
         return fail(GS_ERR_OOM, "counters");
     }
     if (cudaMallocHost(&c->h_counters, sizeof(Counters)) != cudaSuccess ||
-        cudaMallocHost(&c->h_init, sizeof(Counters)) != cudaSuccess) {
+        cudaMallocHost(&c->h_result, sizeof(FrameResult)) != cudaSuccess) {
         if (c->h_counters) cudaFreeHost(c->h_counters);
         c->counters.release();
+        c->classes.release();
         delete c;
         return fail(GS_ERR_OOM, "pinned counters");
     }
-    std::memset(c->h_init, 0, sizeof(Counters));
+    std::memset(c->h_result, 0, sizeof(FrameResult));
     std::memset(c->h_counters, 0, sizeof(Counters));
     for (auto& ev : c->ev) cudaEventCreate(&ev);
     for (auto& ev : c->ev_group) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
@@ -1275,14 +1378,17 @@ int gs_ctx_destroy(gs_ctx* ctx)
     ctx->graphs.clear();
     if (ctx->cap_stream) cudaStreamDestroy(ctx->cap_stream);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
+    if (ctx->raster_stream) cudaStreamDestroy(ctx->raster_stream);
+    if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
+    if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
     DevBuf* bufs[] = {&ctx->views, &ctx->color, &ctx->xy, &ctx->z, &ctx->ell, &ctx->conic, &ctx->rect,
                       &ctx->offsets, &ctx->rec, &ctx->hitmask, &ctx->scan_status, &ctx->view_stats, &ctx->keys0, &ctx->vals0, &ctx->keys1, &ctx->vals1,
                       &ctx->sort_hist, &ctx->sort_status, &ctx->ranges, &ctx->tile_count, &ctx->big_list, &ctx->tile_order,
-                      &ctx->overlaps, &ctx->chunks, &ctx->counters, &ctx->image};
+                      &ctx->overlaps, &ctx->chunks, &ctx->classes, &ctx->counters, &ctx->image};
     for (DevBuf* b : bufs) b->release();
     if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
+    if (ctx->h_result) cudaFreeHost(ctx->h_result);
     if (ctx->h_init) cudaFreeHost(ctx->h_init);
-    if (ctx->h_views) cudaFreeHost(ctx->h_views);
     for (auto& ev : ctx->ev)
         if (ev) cudaEventDestroy(ev);
     for (auto& ev : ctx->ev_group)
@@ -1297,7 +1403,7 @@ int64_t gs_ctx_device_bytes(const gs_ctx* ctx)
     const DevBuf* bufs[] = {&ctx->views, &ctx->color, &ctx->xy, &ctx->z, &ctx->ell, &ctx->conic, &ctx->rect,
                             &ctx->offsets, &ctx->rec, &ctx->hitmask, &ctx->scan_status, &ctx->view_stats, &ctx->keys0, &ctx->vals0, &ctx->keys1, &ctx->vals1,
                             &ctx->sort_hist, &ctx->sort_status, &ctx->ranges, &ctx->tile_count, &ctx->big_list, &ctx->tile_order,
-                      &ctx->overlaps, &ctx->chunks, &ctx->counters, &ctx->image};
+                      &ctx->overlaps, &ctx->chunks, &ctx->classes, &ctx->counters, &ctx->image};
     int64_t t = 0;
     for (const DevBuf* b : bufs) t += (int64_t)b->bytes;
     return t;
@@ -1484,12 +1590,7 @@ int gs_render_host(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cam, con
     const size_t bytes = 4 * (size_t)cam->width * cam->height;
     if (ctx->image.ensure(bytes)) return fail(GS_ERR_OOM, "image");
     uint8_t* outs[1] = {ctx->image.as<uint8_t>()};
-    cudaStream_t st = (cudaStream_t)stream;
-    int rc = run_frame(ctx, scene, cam, 1, *cfg, outs, stats, st);
-    if (rc) return rc;
-    GS_CUDA(cudaMemcpyAsync(h_rgba, ctx->image.p, bytes, cudaMemcpyDeviceToHost, st));
-    GS_CUDA(cudaStreamSynchronize(st));
-    return GS_OK;
+    return run_host_frame(ctx, scene, cam, 1, *cfg, outs, bytes, h_rgba, stats, (cudaStream_t)stream);
 }
 
 int gs_render_batch(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, int32_t num_views,
@@ -1518,38 +1619,16 @@ int gs_render_batch_host(gs_ctx* ctx, const gs_scene* scene, const gs_camera* ca
     std::vector<uint8_t*> outs((size_t)num_views);
     for (int v = 0; v < num_views; ++v) outs[v] = ctx->image.as<uint8_t>() + offs[v];
     cudaStream_t st = (cudaStream_t)stream;
-    if (num_views <= kHostChunkViews) {
-        int rc = run_frame(ctx, scene, cams, num_views, *cfg, outs.data(), stats, st);
-        if (rc) return rc;
-        GS_CUDA(cudaMemcpyAsync(h_rgba, ctx->image.p, total, cudaMemcpyDeviceToHost, st));
-        GS_CUDA(cudaStreamSynchronize(st));
-        return GS_OK;
-    }
-    if (!ctx->copy_stream) GS_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
-    if ((cfg->ordering == GS_ORDER_BUCKETS || cfg->ordering == GS_ORDER_AUTO) && cfg->termination == GS_TERM_TMIN) {
-        // one frame for all views; its raster runs in view groups, each
-        // group read back on the copy stream while the next one renders
-        HostCopy hc;
-        hc.h_rgba = h_rgba;
-        hc.copy = ctx->copy_stream;
-        hc.groups = std::min(kMaxRasterGroups, (num_views + kHostGroupViews - 1) / kHostGroupViews);
-        // the last group's copy is the one nothing overlaps: a quarter of a
-        // group's views, the others share the rest evenly
-        const int last = std::max(1, (num_views + hc.groups - 1) / hc.groups / 4);
-        const int per = (num_views - last + hc.groups - 2) / (hc.groups - 1);
-        for (int g = 0; g < hc.groups; ++g) hc.first_view[g] = std::min(num_views - last, g * per);
-        hc.first_view[hc.groups] = num_views;
-        for (int g = 0; g <= hc.groups; ++g)
-            hc.first_byte[g] = hc.first_view[g] < num_views ? offs[hc.first_view[g]] : total;
-        const int rc = run_frame_bucket(ctx, scene, cams, num_views, *cfg, outs.data(), stats, st, &hc);
-        const cudaError_t se = cudaStreamSynchronize(ctx->copy_stream);
-        if (rc != kSplitViews) {
-            if (rc) return rc;
-            if (se != cudaSuccess) return cuda_fail(se, "image copy");
-            return GS_OK;
-        }
+    const bool buckets = cfg->ordering == GS_ORDER_BUCKETS || cfg->ordering == GS_ORDER_AUTO;
+    if (num_views <= kHostChunkViews)
+        return run_host_frame(ctx, scene, cams, num_views, *cfg, outs.data(), total, h_rgba, stats, st);
+    if (buckets && cfg->termination == GS_TERM_TMIN) {
+        // one frame for all views
+        const int rc = run_grouped_frame(ctx, scene, cams, num_views, *cfg, outs.data(), h_rgba, stats, st);
+        if (rc != kSplitViews) return rc;
         // too many tile keys for one frame: render in chunks below
     }
+    if (!ctx->copy_stream) GS_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
     // Other frames render in chunks of kHostChunkViews views; each chunk's
     // images are copied to the host on a second stream while the next chunk
     // renders (a frame returns with its stream synchronised, so the chunk is
@@ -1648,7 +1727,7 @@ int gs_stage_build(gs_ctx* ctx, int64_t n, const float* d_xy, const float* d_z, 
     int64_t* view_total = ctx->view_stats.as<int64_t>();
     int64_t* view_base = view_total + 1;
     Counters* dc = ctx->counters.as<Counters>();
-    GS_CUDA(cudaMemcpyAsync(ctx->views.p, &v, sizeof(ViewParams), cudaMemcpyHostToDevice, st));
+    GS_CUDA(cudaMemcpyAsync(views_of(ctx), &v, sizeof(ViewParams), cudaMemcpyHostToDevice, st));
     GS_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), st));
     FrameArgs fa = {};
     fa.n = n;
@@ -1657,7 +1736,7 @@ int gs_stage_build(gs_ctx* ctx, int64_t n, const float* d_xy, const float* d_z, 
     fa.views_per_block = 1;
     fa.epoch = take_epochs(ctx->epoch_scan, 1, ctx->scan_status, st);
     fa.num_tiles = blocks;
-    fa.views = ctx->views.as<ViewParams>();
+    fa.views = views_of(ctx);
     fa.xy = (float2*)d_xy;
     fa.ell = (float4*)d_ellipse;
     fa.rect = ctx->rect.as<int2>();
@@ -1680,7 +1759,7 @@ int gs_stage_build(gs_ctx* ctx, int64_t n, const float* d_xy, const float* d_z, 
     EmitArgs ea{};
     ea.n = n;
     ea.num_views = 1;
-    ea.views = ctx->views.as<ViewParams>();
+    ea.views = views_of(ctx);
     ea.offsets = ctx->offsets.as<int32_t>();
     ea.view_total = view_total;
     ea.view_base = view_base;

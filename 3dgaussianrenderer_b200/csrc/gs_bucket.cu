@@ -86,16 +86,25 @@ __device__ __forceinline__ int order_class(const uint32_t count)
     return kOrderClasses - 2 - min(half, kOrderClasses - 2);
 }
 
+// The raster group of a tile.
+__device__ __forceinline__ int group_of(const int64_t* group_tile, const int groups, const int64_t tile)
+{
+    int g = 0;
+    while (g + 1 < groups && group_tile[g + 1] <= tile) ++g;
+    return g;
+}
+
 // ---- 1. tile scan -------------------------------------------------------------
 
-__global__ void __launch_bounds__(kThreads) tile_scan_kernel(TileScanArgs a)
+__global__ void __launch_bounds__(kThreads) tile_scan_kernel(const __grid_constant__ TileScanArgs a)
 {
     constexpr int IPT = kTileScanItems / kThreads;
     __shared__ int64_t s_tmp[kWarps];
     __shared__ int64_t s_base;
     __shared__ int64_t s_blk;
-    __shared__ unsigned int s_class[kOrderClasses];
-    if (threadIdx.x < kOrderClasses) s_class[threadIdx.x] = 0u;
+    __shared__ unsigned int s_class[kMaxRasterGroups * kOrderClasses];
+    const int classes = a.groups * kOrderClasses;
+    for (int k = threadIdx.x; k < classes; k += kThreads) s_class[k] = 0u;
     if (threadIdx.x == 0) s_blk = (int64_t)atomicAdd(a.block_counter, 1ull);
     __syncthreads();
     const int64_t blk = s_blk;
@@ -117,7 +126,7 @@ __global__ void __launch_bounds__(kThreads) tile_scan_kernel(TileScanArgs a)
     for (int j = 0; j < IPT; ++j)
         if (first + j < a.tiles) {
             if (c[j]) a.count[first + j] = 0u;
-            atomicAdd(&s_class[order_class(c[j])], 1u);
+            atomicAdd(&s_class[order_class(c[j]) + kOrderClasses * group_of(a.group_tile, a.groups, first + j)], 1u);
         }
     const int64_t excl = excl_scan_block(sum, s_tmp);
     if (threadIdx.x == kThreads - 1) {
@@ -143,7 +152,8 @@ __global__ void __launch_bounds__(kThreads) tile_scan_kernel(TileScanArgs a)
         }
     }
     __syncthreads();
-    if (threadIdx.x < kOrderClasses && s_class[threadIdx.x]) atomicAdd(&a.class_tiles[threadIdx.x], s_class[threadIdx.x]);
+    for (int k = threadIdx.x; k < classes; k += kThreads)
+        if (s_class[k]) atomicAdd(&a.class_tiles[k], s_class[k]);
     int64_t run = s_base + excl;
     const int64_t cap = a.capacity;
 #pragma unroll
@@ -189,11 +199,17 @@ void launch_tile_scan(const TileScanArgs& a, cudaStream_t st)
 // this one 1.6 ms slower.
 constexpr int kEmitUnroll = 4;
 constexpr int kEmitBlocksPerSm = 4;
-__global__ void __launch_bounds__(kThreads, kEmitBlocksPerSm) emit_bucket_kernel(BucketEmitArgs a)
+__global__ void __launch_bounds__(kThreads, kEmitBlocksPerSm) emit_bucket_kernel(const __grid_constant__ BucketEmitArgs a)
 {
     constexpr int U = kEmitUnroll;
     constexpr int kBatch = kWarps * U;
     __shared__ unsigned long long s_next[2];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        // straight into host memory: a copy at the frame's end would cost its
+        // latency, and nothing after this kernel changes the words
+        *a.result = {*a.total, *a.slot_counter, *a.unit_count, *a.err, *a.overflow};
+        __threadfence_system();
+    }
     if (*a.overflow || *a.err) {
         // some list was too short, so keys of some tiles were never recorded,
         // or the ranges are meaningless: the host redoes or drops the frame,
@@ -208,26 +224,36 @@ __global__ void __launch_bounds__(kThreads, kEmitBlocksPerSm) emit_bucket_kernel
     const int64_t nchunks = (int64_t)(*a.slot_counter >> 32);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (a.order) {
+        // tiles before each (group, class)
         static_assert(kOrderClasses == 32, "one class per lane");
-        int base = (int)a.class_tiles[lane];
-        const int mine = base;
+        __shared__ int s_before[kMaxRasterGroups * kOrderClasses];
+        if (warp == 0) {
+            int carry = 0;
+            for (int g = 0; g < a.groups; ++g) {
+                const int mine = (int)a.class_tiles[g * kOrderClasses + lane];
+                int incl = mine;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(kFull, base, o);
-            if (lane >= o) base += t;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                s_before[g * kOrderClasses + lane] = carry + incl - mine;
+                carry += __shfl_sync(kFull, incl, 31);
+            }
         }
-        base -= mine;  // tiles of the classes before this lane's
+        __syncthreads();
         for (int64_t t0 = ((int64_t)blockIdx.x * kWarps + warp) * 32; t0 < a.tiles; t0 += (int64_t)gridDim.x * kThreads) {
             const int64_t t = t0 + lane;
-            const bool valid = t < a.tiles;
-            const int cls = valid ? order_class((uint32_t)(a.ranges[2 * t + 1] - a.ranges[2 * t])) : kOrderClasses - 1;
-            const unsigned peers = __match_any_sync(kFull, valid ? cls : -1);
+            int cls = -1;
+            if (t < a.tiles)
+                cls = order_class((uint32_t)(a.ranges[2 * t + 1] - a.ranges[2 * t])) +
+                      kOrderClasses * group_of(a.group_tile, a.groups, t);
+            const unsigned peers = __match_any_sync(kFull, cls);
             const int leader = __ffs(peers) - 1;
             unsigned head = 0;
-            if (valid && lane == leader) head = atomicAdd(&a.class_heads[cls], (unsigned)__popc(peers));
+            if (cls >= 0 && lane == leader) head = atomicAdd(&a.class_heads[cls], (unsigned)__popc(peers));
             head = __shfl_sync(kFull, head, leader);
-            const int at = __shfl_sync(kFull, base, cls) + (int)head + __popc(peers & lanemask_lt());
-            if (valid) a.order[at] = (int32_t)t;
+            if (cls >= 0) a.order[s_before[cls] + (int)head + __popc(peers & lanemask_lt())] = (int32_t)t;
         }
     }
     if (threadIdx.x == 0) s_next[0] = atomicAdd(a.batch_counter, (unsigned long long)kBatch);

@@ -117,6 +117,8 @@ struct FrameArgs {
     uint2* overlaps;                   // [32 * chunk_capacity], see BucketEmitArgs
     uint4* chunks;                     // [chunk_capacity]
     int64_t chunk_capacity;
+    unsigned int* zero_words;          // [zero_count] cleared for the kernels that follow
+    int32_t zero_count;
     // splats of more than kLargeCandidates candidate tiles, in units
     uint2* units;                      // [unit_capacity] (slot, unit of the splat)
     unsigned long long* unit_count;    // units listed
@@ -133,6 +135,11 @@ struct FrameArgs {
     float4* probe_color;
 };
 
+// The raster order: half-octave classes of the tiles' key counts; the raster's
+// launches (host-output frames have several).
+constexpr int kOrderClasses = 32;
+constexpr int kMaxRasterGroups = 16;
+
 // The overlap list of a tile-bucket frame, in chunks of 32 places.  Chunk c:
 //   chunks[c] = (mask of the places that hold an overlap, first slot of the
 //                warp that wrote it, its lanes that own a slot, -)
@@ -141,6 +148,15 @@ struct FrameArgs {
 // owner.  A frame whose overlaps need more than chunk_capacity chunks is
 // flagged by the tile scan and redone.
 constexpr int kOverlapTileBits = 27;
+
+// What the host learns of a bucket frame, in pinned memory.
+struct FrameResult {
+    int64_t total;             // K
+    unsigned long long slots;  // slots (low 32 bits) and overlap chunks (high)
+    unsigned long long units;  // units of large splats
+    int err;
+    int overflow;
+};
 
 // Bucket emission: every overlap of slot s is written as
 // (depth bits << 32 | s) at its rank in its tile's range.
@@ -154,11 +170,16 @@ struct BucketEmitArgs {
     int64_t tiles;
     const int* overflow;             // either set: the frame does not stand; all ranges and the big-tile lists
     const int* err;                  // are emptied
+    const int64_t* total;
+    const unsigned long long* unit_count;
+    FrameResult* result;             // out
     unsigned int* big_count;
     unsigned int* huge_count;
     int32_t* order;                  // [tiles] out: the raster order; null: not wanted
-    const unsigned int* class_tiles; // [kOrderClasses] tiles of each class (tile scan)
-    unsigned int* class_heads;       // [kOrderClasses] placed so far; zero at launch
+    int32_t groups;                  // as for the tile scan
+    int64_t group_tile[kMaxRasterGroups];
+    const unsigned int* class_tiles;
+    unsigned int* class_heads;       // [groups * kOrderClasses] placed so far; zero at launch
     uint64_t* keys;
     unsigned long long* batch_counter;  // chunks handed out; zero at launch
 };
@@ -187,9 +208,11 @@ struct TileScanArgs {
     unsigned int* big_count;
     unsigned int* huge_count;
     int32_t fused_cap;
-    unsigned int* class_tiles;       // [kOrderClasses] tiles of each order class; zero at launch
+    // raster order: tiles by group (the raster's launches), in each group by class
+    int32_t groups;
+    int64_t group_tile[kMaxRasterGroups];  // first tile of each group
+    unsigned int* class_tiles;       // [groups * kOrderClasses] tiles of each class; zero at launch
 };
-constexpr int kOrderClasses = 32;
 
 // Per-tile sort of the buckets: each tile's keys are ordered by depth and,
 // among equal depths, by view * n + i, which is the order of a stable sort
@@ -271,7 +294,7 @@ struct RasterArgs {
     int32_t num_views;
     int32_t write_empty;              // 1: tiles without entries are written as (0,0,0,0)
     int64_t num_tiles_total;          // sum of the views' tiles (of this launch's tiles when tile_base is used)
-    int64_t tile_base;                // record raster without `order`: CTA b draws global tile tile_base + b
+    int64_t tile_base;                // CTA b draws global tile order[tile_base + b], or tile_base + b
     const int32_t* ranges;            // [2 * num_tiles_total]
     const int32_t* values;
     const float2* xy;                 // indexed by value (reference-mode kernel)
@@ -287,7 +310,7 @@ struct RasterArgs {
     const uint64_t* keys;
     const int32_t* slot_gi;
     int32_t fused_cap;
-    const int32_t* order;             // non-null: CTA (or queue entry) k rasterises tile order[k]
+    const int32_t* order;             // the raster order of the tiles; null: as numbered
     // record raster (GS_TERM_TMIN) knobs: entries between two tests of whether
     // a block is done (32 or 64), and a persistent grid over the atomic tile queue
     // (tile_counter, zero at launch) instead of one CTA per tile

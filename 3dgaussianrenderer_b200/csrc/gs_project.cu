@@ -579,6 +579,8 @@ __global__ void __launch_bounds__(256, (DEG >= 3 && !FAST) ? 3 : 4) frame_projec
     int gid = i;  // the Gaussian's caller index: equal depths are ordered by it
     if (BUCKET && a.orig) gid = __ldg(&a.orig[at]);
 
+    if (BUCKET && blockIdx.x == 0)
+        for (int k = threadIdx.x; k < a.zero_count; k += 256) a.zero_words[k] = 0u;
     if (DEG >= 0 && threadIdx.x == 0) mbar_init(&s_bar, 1);
     bool sh_asked = DEG < 0 || MANY;  // the coefficients' copy has started (block-uniform) ...
     bool sh_here = sh_asked;          // ... and, as this thread knows, landed

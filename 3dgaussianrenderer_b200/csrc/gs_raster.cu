@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(RefShape<TW, TH>::NT, 640 / RefShape<TW, TH>::
     ts.scan = s_scan;
     ts.red = s_red;
     ts.run = nullptr;
-    const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[blockIdx.x]) : (int64_t)blockIdx.x + a.view0.tile_offset;
+    const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[a.tile_base + blockIdx.x]) : a.tile_base + blockIdx.x;
     const ViewParams& v = view_of_tile(a, gtile);
     raster_ref_tile<TW, TH>(a, v, gtile, (int)(gtile - v.tile_offset), sm, ts);
 }
@@ -697,14 +697,13 @@ __device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64
     }
 }
 
-// One CTA per tile, in the raster order (heavy tiles first) or of the view
-// group [tile_base, tile_base + grid).
+// One CTA per tile of [tile_base, tile_base + grid), in the raster order.
 template <int TW, int TH, int CHUNK>
 __global__ void __launch_bounds__(RecShape<TW, TH>::NT, 640 / RecShape<TW, TH>::NT) raster_rec_kernel(RasterArgs a)
 {
     __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH>)];
     RecSmem<TW, TH>& sm = *reinterpret_cast<RecSmem<TW, TH>*>(smem);
-    const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[blockIdx.x]) : a.tile_base + (int64_t)blockIdx.x;
+    const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[a.tile_base + blockIdx.x]) : a.tile_base + blockIdx.x;
     raster_rec_tile<TW, TH, CHUNK>(a, gtile, sm);
 }
 
@@ -721,7 +720,7 @@ __global__ void __launch_bounds__(RecShape<TW, TH>::NT, 640 / RecShape<TW, TH>::
     for (;;) {
         if (threadIdx.x == 0) {
             const int64_t k = (int64_t)atomicAdd(a.tile_counter, 1ull);
-            s_tile = k < a.num_tiles_total ? (a.order ? (int64_t)__ldg(&a.order[k]) : a.tile_base + k) : -1;
+            s_tile = k < a.num_tiles_total ? (a.order ? (int64_t)__ldg(&a.order[a.tile_base + k]) : a.tile_base + k) : -1;
         }
         __syncthreads();
         const int64_t gtile = s_tile;

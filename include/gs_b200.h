@@ -168,16 +168,15 @@ GS_API int gs_render_host(gs_ctx* ctx, const gs_scene* scene, const gs_camera* c
 
 /* Renders V views (any mix of sizes) of one scene in one batched frame:
  * one flattened tile space with the view in the key's high bits, one
- * persistent rasteriser, replayed as a CUDA graph when the same view set
+ * raster grid, replayed as a CUDA graph when the same view set
  * shape is rendered again.  d_rgba[v] (device) receive 4*W_v*H_v bytes. */
 GS_API int gs_render_batch(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, int32_t num_views,
                     const gs_render_cfg* cfg, uint8_t* const* d_rgba, gs_stats* stats, void* stream);
 /* Same, images copied into one host buffer: view v at byte offset
- * sum_{u<v} 4*W_u*H_u.  Batches of more than 16 views are read back in
- * groups of views while the next group renders: T_min bucket frames render
- * all views in one frame whose raster runs group by group; other frames
- * render 16 views at a time (the stats then add up the frames).  Returns
- * when every image is in h_rgba. */
+ * sum_{u<v} 4*W_u*H_u.  The raster of a bucket frame runs in groups of tile
+ * rows, each read back while the next one renders; onesweep frames, and
+ * reference-mode batches of more than 16 views, render 16 views at a time (the
+ * stats then add up the frames).  Returns when every image is in h_rgba. */
 GS_API int gs_render_batch_host(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, int32_t num_views,
                          const gs_render_cfg* cfg, uint8_t* h_rgba, gs_stats* stats, void* stream);
 
