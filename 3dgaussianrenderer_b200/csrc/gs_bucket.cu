@@ -435,8 +435,10 @@ __device__ void sort_big_count(const TileSortArgs& a, const int64_t start, const
     uint32_t* hist = reinterpret_cast<uint32_t*>(sm.v);
     const bool long_run =
         m <= kBigThreads * 8
-            ? tilesort::count_sort_tile<kBigThreads, 8>(a.keys + start, m, a.slot_gi, sm, hist, a.vals + start)
-            : tilesort::count_sort_tile<kBigThreads, 0>(a.keys + start, m, a.slot_gi, sm, hist, a.vals + start);
+            ? tilesort::count_sort_tile<kBigThreads, 8>(a.keys + start, m, a.slot_gi, sm, hist, a.vals + start,
+                                                         kTileSortSmemKeys)
+            : tilesort::count_sort_tile<kBigThreads, 0>(a.keys + start, m, a.slot_gi, sm, hist, a.vals + start,
+                                                         kTileSortSmemKeys);
     if (!long_run) return;
     if (m <= 2048)
         sort_big_smem<8>(a, start, m, sm);
@@ -482,8 +484,8 @@ __global__ void __launch_bounds__(kBigThreads, kBigBlocksPerSm) tile_sort_big_ke
 
 // The tiles above kTileSortSmemKeys keys, by persistent 1024-thread CTAs
 // (one per SM: 128 KB of keys and a 64 KB histogram of 2^15 bins in shared
-// memory), in the counting form over 15 depth bits.  A tile above
-// kTileSortHugeKeys keys, or with a run longer than kMaxRankRun, is handed
+// memory), in the counting form over 15 depth bits, above kTileSortHugeKeys
+// keys in parts.  A tile above kTileSortHugeMax keys, or with a run longer than kMaxRankRun, is handed
 // to tile_sort_big_kernel: appended to its list, which that kernel, launched
 // after this one on the same stream, reads when it starts.
 constexpr int kHugeThreads = 1024;
@@ -504,10 +506,13 @@ __global__ void __launch_bounds__(kHugeThreads, 1) tile_sort_huge_kernel(TileSor
         const int64_t t = a.big_list[a.tiles + j];
         const int64_t start = __ldg(&a.ranges[2 * t]);
         const int m = __ldg(&a.ranges[2 * t + 1]) - (int)start;
-        bool handed = m > kTileSortHugeKeys;
-        if (!handed)
+        bool handed = m > kTileSortHugeMax;
+        if (!handed && m <= kTileSortHugeKeys)
+            handed = tilesort::count_sort_tile<kHugeThreads, kTileSortHugeKeys / kHugeThreads, kHugeBits>(
+                a.keys + start, m, a.slot_gi, sm, hist, a.vals + start, kTileSortHugeKeys);
+        else if (!handed)
             handed = tilesort::count_sort_tile<kHugeThreads, 0, kHugeBits>(a.keys + start, m, a.slot_gi, sm, hist,
-                                                                          a.vals + start);
+                                                                          a.vals + start, kTileSortHugeKeys);
         if (handed && threadIdx.x == 0) a.big_list[atomicAdd(a.big_count, 1u)] = (int32_t)t;
         __syncthreads();  // shared memory is reused by the next tile
     }

@@ -232,10 +232,11 @@ struct TileSortArgs {
     int32_t prefix_bits;             // depth bits the radix passes sort (8..32; 0 = 16)
 };
 constexpr int kTileSortSmemKeys = 4096;
-// Tiles of up to this many keys are sorted in the shared memory of one
-// 1024-thread CTA (tile_sort_huge_kernel); larger ones by passes through
-// global memory.
+// Tiles of up to kTileSortHugeMax keys (16-bit counters) are sorted in the
+// shared memory of one 1024-thread CTA (tile_sort_huge_kernel), which holds
+// kTileSortHugeKeys at a time; larger ones by passes through global memory.
 constexpr int kTileSortHugeKeys = 16384;
+constexpr int kTileSortHugeMax = 65535;
 // Keys a tile may have to be sorted inside its raster CTA (8 per two
 // pixels); larger tiles are sorted ahead of the raster.
 constexpr int kFusedIpt = 8;

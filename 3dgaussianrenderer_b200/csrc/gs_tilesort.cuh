@@ -314,8 +314,8 @@ __device__ void sort_tile(const uint64_t* __restrict__ keys, const int m, const 
 }
 
 // Counting-sort form of sort_tile for the stand-alone sort of the larger
-// tiles (m keys, as many as sm.k holds; NT threads), writing the tile's
-// slots in (depth, index) order to `out`.  One pass places every key in
+// tiles (m < 2^16 keys, `cap` of which sm.k holds; NT threads), writing the
+// tile's slots in (depth, index) order to `out`.  One pass places every key in
 // shared memory by the top BITS varying depth bits: a histogram of 16-bit
 // counters packed two to a word (`hist`, 2^(BITS - 1) words; counts and
 // offsets stay below 2^16, so m < 2^16), its exclusive scan, then each key
@@ -329,8 +329,10 @@ __device__ void sort_tile(const uint64_t* __restrict__ keys, const int m, const 
 // costs L comparisons per key, in parallel.  The callers keep about two
 // bins per key (13 bits for up to 4096 keys, 15 for up to 16384); at 13
 // bits no run on the benchmark's views is longer than 25 keys.
-// IPT > 0: m <= NT * IPT, each thread holds its IPT keys in registers
-// across the passes; IPT = 0: every pass reads the keys from global memory.
+// IPT > 0: m <= NT * IPT <= cap, each thread holds its IPT keys in registers
+// across the passes, loaded all at once; IPT = 0: every pass reads the keys
+// from global memory, and a tile of more than cap keys is placed and ranked in
+// parts of whole bins that fit.
 // Returns true when some run is longer than kMaxRankRun (`out` then holds
 // only part of the order); the caller then sorts the tile another way.
 // Every thread of the CTA must call it; it ends with a barrier.
@@ -339,7 +341,7 @@ constexpr int kMaxRankRun = 64;
 
 template <int NT, int IPT, int BITS = kCountBits>
 __device__ bool count_sort_tile(const uint64_t* __restrict__ keys, const int m, const int32_t* __restrict__ slot_gi,
-                                const Smem& sm, uint32_t* hist, int32_t* __restrict__ out)
+                                const Smem& sm, uint32_t* hist, int32_t* __restrict__ out, const int cap)
 {
     constexpr int NW = NT / 32;
     constexpr int kBins = 1 << BITS;
@@ -360,6 +362,7 @@ __device__ bool count_sort_tile(const uint64_t* __restrict__ keys, const int m, 
             }
         }
     } else {
+#pragma unroll 4
         for (int p = threadIdx.x; p < m; p += NT) {
             const uint64_t k = keys[p];
             o |= k;
@@ -379,6 +382,7 @@ __device__ bool count_sort_tile(const uint64_t* __restrict__ keys, const int m, 
         for (int i = 0; i < IPT; ++i)
             if (i * NT + (int)threadIdx.x < m) count(kr[i]);
     } else {
+#pragma unroll 4
         for (int p = threadIdx.x; p < m; p += NT) count(keys[p]);
     }
     __syncthreads();
@@ -407,33 +411,58 @@ __device__ bool count_sort_tile(const uint64_t* __restrict__ keys, const int m, 
     if (wbase)
         for (int r = 0; r < WPW / 32; ++r) hist[warp * WPW + r * 32 + lane] += (uint32_t)wbase | ((uint32_t)wbase << 16);
     __syncthreads();
-    auto place = [&](const uint64_t k) {
-        const uint32_t d = (uint32_t)(k >> shift) & (kBins - 1);
-        const uint32_t half = (d & 1u) << 4;
-        const uint32_t old = atomicAdd(&hist[d >> 1], 1u << half);
-        sm.k[(old >> half) & 0xFFFFu] = k;
-    };
-    if constexpr (IPT > 0) {
-#pragma unroll
-        for (int i = 0; i < IPT; ++i)
-            if (i * NT + (int)threadIdx.x < m) place(kr[i]);
-    } else {
-        for (int p = threadIdx.x; p < m; p += NT) place(keys[p]);
-    }
-    __syncthreads();
+    // the parts: bins [b0, b1) hold the keys of positions [s0, s0 + cnt)
     bool too_long = false;
-    for (int p = threadIdx.x; p < m; p += NT) {
-        const uint64_t k = sm.k[p];
-        const uint32_t d = (uint32_t)(k >> shift) & (kBins - 1);
-        const uint32_t e = (hist[d >> 1] >> ((d & 1u) << 4)) & 0xFFFFu;
-        const uint32_t s0 = d ? (hist[(d - 1) >> 1] >> (((d - 1) & 1u) << 4)) & 0xFFFFu : 0u;
-        if (e - s0 > (uint32_t)kMaxRankRun) {
-            too_long = true;
-            continue;
+    for (int b0 = 0, s0 = 0; s0 < m;) {
+        int b1 = kBins, cnt = m - s0;
+        if (IPT == 0 && cnt > cap) {
+            // the last bin whose keys still fit: starts only rise
+            auto start = [&](const int d) { return (int)((hist[d >> 1] >> ((d & 1) << 4)) & 0xFFFFu); };
+            int lo = b0, hi = kBins - 1;  // start(lo) - s0 <= cap
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (start(mid) - s0 <= cap)
+                    lo = mid;
+                else
+                    hi = mid - 1;
+            }
+            b1 = lo;
+            cnt = start(b1) - s0;
+            if (cnt == 0) return true;  // one bin has more than cap keys (uniform: every thread reads the same)
+            __syncthreads();            // starts are read before the placement moves them
         }
-        uint32_t rank = 0;
-        for (uint32_t q = s0; q < e; ++q) rank += key_before(sm.k[q], k, slot_gi) ? 1u : 0u;
-        out[s0 + rank] = (int32_t)(uint32_t)k;
+        auto place = [&](const uint64_t k) {
+            const uint32_t d = (uint32_t)(k >> shift) & (kBins - 1);
+            if (IPT == 0 && (d < (uint32_t)b0 || d >= (uint32_t)b1)) return;
+            const uint32_t half = (d & 1u) << 4;
+            const uint32_t old = atomicAdd(&hist[d >> 1], 1u << half);
+            sm.k[(int)((old >> half) & 0xFFFFu) - s0] = k;
+        };
+        if constexpr (IPT > 0) {
+#pragma unroll
+            for (int i = 0; i < IPT; ++i)
+                if (i * NT + (int)threadIdx.x < m) place(kr[i]);
+        } else {
+#pragma unroll 4
+            for (int p = threadIdx.x; p < m; p += NT) place(keys[p]);
+        }
+        __syncthreads();
+        for (int p = threadIdx.x; p < cnt; p += NT) {
+            const uint64_t k = sm.k[p];
+            const uint32_t d = (uint32_t)(k >> shift) & (kBins - 1);
+            const int e = (int)((hist[d >> 1] >> ((d & 1u) << 4)) & 0xFFFFu) - s0;
+            const int f = d ? max((int)((hist[(d - 1) >> 1] >> (((d - 1) & 1u) << 4)) & 0xFFFFu) - s0, 0) : 0;
+            if (e - f > kMaxRankRun) {
+                too_long = true;
+                continue;
+            }
+            int rank = 0;
+            for (int q = f; q < e; ++q) rank += key_before(sm.k[q], k, slot_gi) ? 1 : 0;
+            out[s0 + f + rank] = (int32_t)(uint32_t)k;
+        }
+        b0 = b1;
+        s0 += cnt;
+        if (s0 < m) __syncthreads();  // the keys give way to the next part's
     }
     return __syncthreads_or(too_long) != 0;
 }
