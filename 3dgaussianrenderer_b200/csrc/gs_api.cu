@@ -153,6 +153,11 @@ constexpr int kHostChunkViews = 16;
 // takes 36 us at 55 GB/s, several times its launch and its group's.
 constexpr size_t kHostGroupBytes = 2u << 20;
 
+// The raster's last CTAs that stamp its end: enough that the last one to finish
+// is among them (the order puts the long ones first), few enough that their
+// writes to host memory do not hold up the images' copies.
+constexpr int64_t kStampCtas = 2048;
+
 // Host read-back overlapped with the frame (bucket frames): the raster runs in
 // groups of tile rows, one after the other in image order, each group's end is
 // marked by an event, and its part of the images is copied on `copy` after it.
@@ -262,7 +267,7 @@ struct gs_ctx {
     Counters* h_init = nullptr;            // pinned image of `views`: the reset counters, then
     ViewParams* h_views = nullptr;         // the view parameters at kViewsOffset
     int h_views_cap = 0;
-    cudaEvent_t ev[8] = {};
+    cudaEvent_t ev[8] = {};                // onesweep frames' stages [0, 6), the sort probe's [6, 8)
     int64_t key_capacity = 0;
     cudaStream_t cap_stream = nullptr;     // graph capture
     cudaStream_t copy_stream = nullptr;    // image read-back of the host-output batches
@@ -707,7 +712,6 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
         GS_CUDA(cudaMemsetAsync(ctx->tile_count.p, 0, ctx->tile_count.bytes, st));
         if (!capturing) ctx->tile_count_dirty = false;
     }
-    GS_CUDA(record(ctx->ev[0], st, capturing));
 
     FrameArgs fa{};
     fa.n = p.n;
@@ -749,6 +753,7 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
         fa.probe_conic = reinterpret_cast<float4*>(p.probe->d_conic);
         fa.probe_color = reinterpret_cast<float4*>(p.probe->d_color);
     }
+    fa.result = ctx->h_result;
     fa.zero_words = ctx->classes.as<unsigned int>();
     fa.zero_count = 2 * kMaxRasterGroups * kOrderClasses;
     if (p.n > 0) {
@@ -781,7 +786,6 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ta.groups = in_groups ? p.host_copy->groups : 1;
     for (int g = 0; g < ta.groups; ++g) ta.group_tile[g] = in_groups ? p.host_copy->first_tile[g] : 0;
     launch_tile_scan(ta, st);
-    GS_CUDA(record(ctx->ev[1], st, capturing));
 
     BucketEmitArgs ea{};
     ea.slot_counter = &dc->slots;
@@ -806,7 +810,6 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ea.keys = ctx->keys0.as<uint64_t>();
     ea.batch_counter = &dc->emit_batch;
     launch_emit_bucket(ea, ctx->num_sms, st);
-    GS_CUDA(record(ctx->ev[3], st, capturing));
 
     TileSortArgs sa{};
     sa.ranges = ctx->ranges.as<int32_t>();
@@ -820,8 +823,8 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     sa.big_count = &dc->big_tiles;
     sa.huge_count = &dc->huge_tiles;
     sa.prefix_bits = cfg.sort_bits;
+    sa.result = ctx->h_result;
     if (p.n > 0) launch_tile_sort(sa, ctx->num_sms, st);
-    GS_CUDA(record(ctx->ev[4], st, capturing));
 
     RasterArgs ra{};
     ra.view0 = ctx->h_views[0];
@@ -841,6 +844,9 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ra.slot_gi = ctx->offsets.as<int32_t>();
     ra.fused_cap = fused_tile_capacity(cfg.tile_w, cfg.tile_h);
     ra.order = ea.order;
+    ra.result = ctx->h_result;
+    ra.start_from = 1;
+    ra.end_from = ra.num_tiles_total - kStampCtas;
     ra.rec_chunk = cfg.raster_chunk;
     ra.rec_persistent = cfg.raster_persistent;
     ra.sort_prefix_bits = cfg.sort_bits;
@@ -860,6 +866,8 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
             RasterArgs rg = ra;
             rg.tile_base = hc.first_tile[g];
             rg.num_tiles_total = hc.first_tile[g + 1] - hc.first_tile[g];
+            rg.start_from = g == 0 ? 1 : 0;
+            rg.end_from = g + 2 >= hc.groups ? rg.num_tiles_total - kStampCtas : rg.num_tiles_total;
             // a persistent group launch starts its own queue from zero
             if (rg.rec_persistent) GS_CUDA(cudaMemsetAsync(&dc->raster_tile, 0, sizeof(unsigned long long), gst));
             launch_raster(rg, cfg.tile_w, cfg.tile_h, cfg.termination, ctx->num_sms, gst);
@@ -873,7 +881,6 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
         launch_raster(ra, cfg.tile_w, cfg.tile_h, cfg.termination, ctx->num_sms, st);
     }
     GS_CUDA(cudaGetLastError());
-    GS_CUDA(record(ctx->ev[5], st, capturing));
     return GS_OK;
 }
 
@@ -1050,11 +1057,16 @@ int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, 
     ctx->last_fused_cap = fused_tile_capacity(cfg.tile_w, cfg.tile_h);
     if (stats) {
         stats->sh_eval_ms = 0.0;
-        stats->project_ms = ms_between(ctx->ev[0], ctx->ev[1]);
-        stats->build_tile_ms = ms_between(ctx->ev[1], ctx->ev[3]);
-        stats->sort_ms = ms_between(ctx->ev[3], ctx->ev[4]);  // the tiles too big for the raster CTAs
-        stats->raster_ms = ms_between(ctx->ev[4], ctx->ev[5]);
-        stats->total_ms = ms_between(ctx->ev[0], ctx->ev[5]);
+        // without Gaussians only the emission and the raster run
+        unsigned long long t[kFrameTimes];
+        std::copy(ctx->h_result->t, ctx->h_result->t + kFrameTimes, t);
+        if (p.n == 0) t[kTimeStart] = t[kTimeSort] = t[kTimeEmit];
+        auto ms = [&](FrameTime a, FrameTime b) { return t[b] > t[a] ? (double)(t[b] - t[a]) * 1e-6 : 0.0; };
+        stats->project_ms = ms(kTimeStart, kTimeEmit);
+        stats->build_tile_ms = ms(kTimeEmit, kTimeSort);
+        stats->sort_ms = ms(kTimeSort, kTimeRaster);  // the tiles too big for the raster CTAs
+        stats->raster_ms = ms(kTimeRaster, kTimeEnd);
+        stats->total_ms = ms(kTimeStart, kTimeEnd);
         stats->num_keys = ctx->h_result->total;
         stats->num_tiles = p.tiles_total;
         // frame kernel, large splats, the two big-tile sorts; tile scan, bucket emit,

@@ -207,8 +207,12 @@ __global__ void __launch_bounds__(kThreads, kEmitBlocksPerSm) emit_bucket_kernel
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // straight into host memory: a copy at the frame's end would cost its
         // latency, and nothing after this kernel changes the words
-        *a.result = {*a.total, *a.slot_counter, *a.unit_count, *a.err, *a.overflow};
-        __threadfence_system();
+        stamp(a.result, kTimeEmit);
+        a.result->total = *a.total;
+        a.result->slots = *a.slot_counter;
+        a.result->units = *a.unit_count;
+        a.result->err = *a.err;
+        a.result->overflow = *a.overflow;
     }
     if (*a.overflow || *a.err) {
         // some list was too short, so keys of some tiles were never recorded,
@@ -501,6 +505,7 @@ __global__ void __launch_bounds__(kHugeThreads, 1) tile_sort_huge_kernel(TileSor
     sm.scan = s_scan;
     sm.red = s_red;
     uint32_t* hist = reinterpret_cast<uint32_t*>(smem + kTileSortHugeKeys * 8);
+    if (blockIdx.x == 0 && threadIdx.x == 0) stamp(a.result, kTimeSort);
     const int nhuge = (int)*a.huge_count;
     for (int j = blockIdx.x; j < nhuge; j += gridDim.x) {
         const int64_t t = a.big_list[a.tiles + j];

@@ -61,6 +61,27 @@ inline int device_sm_count()
     return sms;
 }
 
+// What the host learns of a bucket frame, in pinned memory that the kernels
+// write: the emission the counts, and the times (globaltimer, ns) the kernels
+// at the stages' ends.  Events between the stages, whose records a graph runs
+// as nodes of their own, cost a frame 22 us of wall time.
+enum FrameTime { kTimeStart, kTimeEmit, kTimeSort, kTimeRaster, kTimeEnd, kFrameTimes };
+struct FrameResult {
+    unsigned long long t[kFrameTimes];
+    int64_t total;             // K
+    unsigned long long slots;  // slots (low 32 bits) and overlap chunks (high)
+    unsigned long long units;  // units of large splats
+    int err;
+    int overflow;
+};
+
+__device__ __forceinline__ void stamp(FrameResult* r, const FrameTime k)
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    r->t[k] = t;
+}
+
 // Splats of more than kLargeCandidates candidate tiles are walked by
 // large_overlap_kernel, kUnitCandidates at a time (a threshold of 64 takes 7.2
 // instead of 8.0 ms for both kernels on the 4K view of 10M large splats, but
@@ -117,6 +138,7 @@ struct FrameArgs {
     uint2* overlaps;                   // [32 * chunk_capacity], see BucketEmitArgs
     uint4* chunks;                     // [chunk_capacity]
     int64_t chunk_capacity;
+    FrameResult* result;               // out: the frame's start
     unsigned int* zero_words;          // [zero_count] cleared for the kernels that follow
     int32_t zero_count;
     // splats of more than kLargeCandidates candidate tiles, in units
@@ -149,15 +171,6 @@ constexpr int kMaxRasterGroups = 16;
 // flagged by the tile scan and redone.
 constexpr int kOverlapTileBits = 27;
 
-// What the host learns of a bucket frame, in pinned memory.
-struct FrameResult {
-    int64_t total;             // K
-    unsigned long long slots;  // slots (low 32 bits) and overlap chunks (high)
-    unsigned long long units;  // units of large splats
-    int err;
-    int overflow;
-};
-
 // Bucket emission: every overlap of slot s is written as
 // (depth bits << 32 | s) at its rank in its tile's range.
 struct BucketEmitArgs {
@@ -172,7 +185,7 @@ struct BucketEmitArgs {
     const int* err;                  // are emptied
     const int64_t* total;
     const unsigned long long* unit_count;
-    FrameResult* result;             // out
+    FrameResult* result;             // out: all but the frame's and the sort's and raster's times
     unsigned int* big_count;
     unsigned int* huge_count;
     int32_t* order;                  // [tiles] out: the raster order; null: not wanted
@@ -230,6 +243,7 @@ struct TileSortArgs {
     unsigned int* big_count;
     const unsigned int* huge_count;
     int32_t prefix_bits;             // depth bits the radix passes sort (8..32; 0 = 16)
+    FrameResult* result;             // out: the sort's start
 };
 constexpr int kTileSortSmemKeys = 4096;
 // Tiles of up to kTileSortHugeMax keys (16-bit counters) are sorted in the
@@ -315,6 +329,8 @@ struct RasterArgs {
     // record raster (GS_TERM_TMIN) knobs: entries between two tests of whether
     // a block is done (32 or 64), and a persistent grid over the atomic tile queue
     // (tile_counter, zero at launch) instead of one CTA per tile
+    FrameResult* result;              // out: the raster's times; null: not wanted
+    int64_t start_from, end_from;     // CTAs before start_from stamp its start, those from end_from on its end
     int32_t rec_chunk;
     int32_t rec_persistent;
     int32_t sort_prefix_bits;         // depth bits the fused tile sort radix-sorts (8..32; 0 = 16)

@@ -421,15 +421,26 @@ __global__ void __launch_bounds__(256) large_overlap_kernel(const __grid_constan
             const int left = w.total - 32 * lane;
             a.chunks[first + lane] = make_uint4(left >= 32 ? kFull : (1u << left) - 1u, slot, 0u, 0u);
         }
-        for (int s = 0; s < steps; ++s) {
-            const unsigned bal = __shfl_sync(kFull, mine, s);
-            const int at = __shfl_sync(kFull, w.excl, s);
-            if (!((bal >> lane) & 1u)) continue;
-            int lx, ly;
-            divmod_small(c0 + 32 * s + lane, r.z, ly, lx);
-            const uint32_t gt = (uint32_t)v.tile_offset + (uint32_t)((r.y + ly) * v.tiles_x + r.x + lx);
-            const uint32_t rank = atomicAdd(&a.tile_count[gt], 1u);
-            if (room) a.overlaps[first * 32 + at + __popc(bal & lanemask_lt())] = make_uint2(gt, rank);
+        for (int s0 = 0; s0 < steps; s0 += 4) {
+            uint2 x[4];
+            int at[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int s = s0 + u;
+                const unsigned bal = s < steps ? __shfl_sync(kFull, mine, s & 31) : 0u;
+                at[u] = __shfl_sync(kFull, w.excl, s & 31) + __popc(bal & lanemask_lt());
+                if (!((bal >> lane) & 1u)) {
+                    at[u] = -1;
+                    continue;
+                }
+                int lx, ly;
+                divmod_small(c0 + 32 * s + lane, r.z, ly, lx);
+                x[u].x = (uint32_t)v.tile_offset + (uint32_t)((r.y + ly) * v.tiles_x + r.x + lx);
+                x[u].y = atomicAdd(&a.tile_count[x[u].x], 1u);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (room && at[u] >= 0) a.overlaps[first * 32 + at[u]] = x[u];
         }
     }
 }
@@ -579,6 +590,7 @@ __global__ void __launch_bounds__(256, (DEG >= 3 && !FAST) ? 3 : 4) frame_projec
     int gid = i;  // the Gaussian's caller index: equal depths are ordered by it
     if (BUCKET && a.orig) gid = __ldg(&a.orig[at]);
 
+    if (BUCKET && blockIdx.x == 0 && threadIdx.x == 0) stamp(a.result, kTimeStart);
     if (BUCKET && blockIdx.x == 0)
         for (int k = threadIdx.x; k < a.zero_count; k += 256) a.zero_words[k] = 0u;
     if (DEG >= 0 && threadIdx.x == 0) mbar_init(&s_bar, 1);
@@ -619,11 +631,11 @@ __global__ void __launch_bounds__(256, (DEG >= 3 && !FAST) ? 3 : 4) frame_projec
         if (valid) {
             // outside the frustum: culled, no tile (whole warps of a
             // spatially ordered scene skip the projection together)
-            const float4 p = MANY ? kept_p : reload(&a.pos[at]);
+            const float4 p = MANY ? kept_p : reload(&a.pos[at]), sr = MANY ? kept_sr : reload(&a.sr[at]);
             const ViewPos w = view_position<FAST>(p, v);
             if (in_frustum(w)) {
                 projected = true;
-                s = project_gaussian<FAST>(w, MANY ? kept_sr : reload(&a.sr[at]), v);
+                s = project_gaussian<FAST>(w, sr, v);
                 e = {s.x, s.y, s.cs, s.sn, s.ex, s.ey};
                 r = tile_rect(e, v);
                 cand = rect_candidates(r);

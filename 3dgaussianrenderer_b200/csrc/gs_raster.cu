@@ -212,6 +212,17 @@ __device__ __forceinline__ int slot_at(const RasterArgs& a, const uint64_t* sk, 
     return sk ? (int)(uint32_t)sk[idx] : __ldg(&a.values[first + idx]);
 }
 
+// The raster's times: its first CTA the start, every warp of the last CTAs the
+// end (the last writer stays).
+__device__ __forceinline__ void stamp_start(const RasterArgs& a)
+{
+    if (a.result && blockIdx.x < a.start_from && threadIdx.x == 0) stamp(a.result, kTimeRaster);
+}
+__device__ __forceinline__ void stamp_end(const RasterArgs& a)
+{
+    if (a.result && blockIdx.x >= a.end_from && (threadIdx.x & 31) == 0) stamp(a.result, kTimeEnd);
+}
+
 // The view a global tile belongs to: binary search over the views' first tiles.
 __device__ __forceinline__ const ViewParams& view_of_tile(const RasterArgs& a, const int64_t gtile)
 {
@@ -435,7 +446,9 @@ __global__ void __launch_bounds__(RefShape<TW, TH>::NT, 640 / RefShape<TW, TH>::
     ts.run = nullptr;
     const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[a.tile_base + blockIdx.x]) : a.tile_base + blockIdx.x;
     const ViewParams& v = view_of_tile(a, gtile);
+    stamp_start(a);
     raster_ref_tile<TW, TH>(a, v, gtile, (int)(gtile - v.tile_offset), sm, ts);
+    stamp_end(a);
 }
 
 template <int TW, int TH>
@@ -704,7 +717,9 @@ __global__ void __launch_bounds__(RecShape<TW, TH>::NT, 640 / RecShape<TW, TH>::
     __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH>)];
     RecSmem<TW, TH>& sm = *reinterpret_cast<RecSmem<TW, TH>*>(smem);
     const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[a.tile_base + blockIdx.x]) : a.tile_base + blockIdx.x;
+    stamp_start(a);
     raster_rec_tile<TW, TH, CHUNK>(a, gtile, sm);
+    stamp_end(a);
 }
 
 // Persistent CTAs (as many as fit on the SMs at once) that pull tiles from
@@ -717,6 +732,7 @@ __global__ void __launch_bounds__(RecShape<TW, TH>::NT, 640 / RecShape<TW, TH>::
     __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH>)];
     RecSmem<TW, TH>& sm = *reinterpret_cast<RecSmem<TW, TH>*>(smem);
     __shared__ int64_t s_tile;
+    stamp_start(a);
     for (;;) {
         if (threadIdx.x == 0) {
             const int64_t k = (int64_t)atomicAdd(a.tile_counter, 1ull);
@@ -724,10 +740,11 @@ __global__ void __launch_bounds__(RecShape<TW, TH>::NT, 640 / RecShape<TW, TH>::
         }
         __syncthreads();
         const int64_t gtile = s_tile;
-        if (gtile < 0) return;
+        if (gtile < 0) break;
         raster_rec_tile<TW, TH, CHUNK>(a, gtile, sm);
         __syncthreads();  // s_tile and the sort's shared memory are reused
     }
+    stamp_end(a);
 }
 
 template <int TW, int TH, int CHUNK>
