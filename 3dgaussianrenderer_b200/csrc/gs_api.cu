@@ -354,11 +354,15 @@ cudaError_t record(cudaEvent_t ev, cudaStream_t st, bool capturing)
     return capturing ? cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal) : cudaEventRecord(ev, st);
 }
 
-// Onesweep tile shape of the stage sort: 8192-key tiles up to 16M keys (on
-// the 2.6M keys of a 1024^2 frame they cut the look-back chain to a wave:
-// 0.253 against 0.258 ms with 4096-key tiles), the default shape above
-// (17.1 against 17.5 ms on 222M keys).
-int stage_sort_variant(int64_t num_keys) { return num_keys <= (1ll << 24) ? 3 : 0; }
+// Onesweep tile shape of the stage sort: 4096-key tiles while they are one wave
+// (2 blocks per SM: 50k keys take 69 against 88 us), 8192-key tiles up to 16M
+// keys (they cut the look-back chain: 1.4M keys 176 against 191 us, 2.4M keys
+// 203 against 242 us), the default shape above (100M keys 7.2 against 7.7 ms).
+int stage_sort_variant(int64_t num_keys, int num_sms)
+{
+    if (num_keys <= 2ll * num_sms * kSortTile) return 0;
+    return num_keys <= (1ll << 24) ? 3 : 0;
+}
 
 int ensure_sort_scratch(gs_ctx* ctx, int64_t num_items)
 {
@@ -1816,7 +1820,7 @@ int gs_stage_sort(gs_ctx* ctx, int64_t num_keys, int32_t key_bits, uint64_t* d_k
     const uint32_t ep = take_epochs(ctx->epoch_sort, (uint32_t)sort_passes(key_bits), ctx->sort_status, st);
     const int passes =
         launch_sort(d_keys, d_values, d_keys_alt, d_values_alt, num_keys, nullptr, key_bits, ss, ep, ctx->num_sms, st,
-                    stage_sort_variant(num_keys));
+                    stage_sort_variant(num_keys, ctx->num_sms));
     GS_CUDA(cudaGetLastError());
     GS_CUDA(cudaMemcpyAsync(&ctx->h_counters->err, &dc->err, sizeof(int), cudaMemcpyDeviceToHost, st));
     GS_CUDA(cudaStreamSynchronize(st));
@@ -1858,7 +1862,7 @@ int gs_probe_sort_timed(gs_ctx* ctx, int64_t num_keys, int32_t key_bits, const u
         const uint32_t ep = take_epochs(ctx->epoch_sort, (uint32_t)sort_passes(key_bits), ctx->sort_status, st);
         GS_CUDA(cudaEventRecord(ctx->ev[6], st));
         passes = launch_sort(d_keys, d_values, d_keys_alt, d_values_alt, num_keys, nullptr, key_bits, ss, ep,
-                             ctx->num_sms, st, stage_sort_variant(num_keys));
+                             ctx->num_sms, st, stage_sort_variant(num_keys, ctx->num_sms));
         GS_CUDA(cudaGetLastError());
         GS_CUDA(cudaEventRecord(ctx->ev[7], st));
         GS_CUDA(cudaMemcpyAsync(&ctx->h_counters->err, &dc->err, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -717,9 +717,12 @@ __device__ __forceinline__ int load_flag(const int* p)
 
 // Exclusive prefix of `tile`'s aggregate over all earlier tiles, walking
 // back through status[tile-1], status[tile-2], ... (`stride` words apart).
+// kLookBack words are read at a time: a walk past the aggregates of the tiles in
+// flight is then a few L2 latencies long instead of one per tile.
 // Gives up after kSpinLimit polls, or as soon as another block has
 // reported an error, setting *err; the result is then meaningless and the
 // host discards the frame.
+constexpr int kLookBack = 8;
 __device__ __forceinline__ uint64_t look_back(const uint64_t* status, const int64_t tile, const int64_t stride,
                                               const uint32_t epoch, int* err, const int err_code,
                                               const int spin_limit = kSpinLimit)
@@ -729,18 +732,27 @@ __device__ __forceinline__ uint64_t look_back(const uint64_t* status, const int6
     int64_t j = tile - 1;
     int spins = 0;
     while (j >= 0) {
-        const uint64_t s = load_status(status + j * stride);
-        if ((s & (kFlagP | kFlagA)) == 0 || (s & kEpochMask) != want) {
+        uint64_t s[kLookBack];
+#pragma unroll
+        for (int u = 0; u < kLookBack; ++u)
+            s[u] = j - u >= 0 ? load_status(status + (j - u) * stride) : (kFlagP | want);  // nothing before tile 0
+        int taken = 0;
+#pragma unroll
+        for (int u = 0; u < kLookBack; ++u) {
+            if (taken < u) break;
+            if ((s[u] & (kFlagP | kFlagA)) == 0 || (s[u] & kEpochMask) != want) break;
+            excl += s[u] & kValueMask;
+            if (s[u] & kFlagP) return excl;
+            taken = u + 1;
+        }
+        j -= taken;
+        if (taken == 0) {
             if (++spins > spin_limit || load_flag(err) != 0) {
                 atomicCAS(err, 0, err_code);
                 return excl;
             }
             if (spins > 64) __nanosleep(32);
-            continue;
         }
-        excl += s & kValueMask;
-        if (s & kFlagP) break;
-        --j;
     }
     return excl;
 }
