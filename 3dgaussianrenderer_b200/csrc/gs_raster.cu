@@ -268,9 +268,10 @@ struct RefSmem {
 
 // Pixel layout of a tile: 8 lanes across, so a warp covers 8 NC x 8 pixels
 // (a lane's two rows are 4 apart).
-template <int TW, int TH>
+template <int TW, int TH, int COLS>
 struct RefShape {
-    static constexpr int NC = TW / 8;
+    static constexpr int NC = COLS;
+    static constexpr int WX = TW / (8 * NC);  // warps across a tile
     static constexpr int NT = TW * TH / (2 * NC);
     static constexpr int CAP = TW * TH / 2 * kFusedIpt;
 };
@@ -330,19 +331,20 @@ __device__ __forceinline__ bool wild_entry(const RefSmem& sm, const int j)
              fabsf(k.z) < 1e30f);
 }
 
-template <int TW, int TH>
+template <int TW, int TH, int COLS>
 __device__ __forceinline__ void raster_ref_tile(const RasterArgs& a, const ViewParams& v, const int64_t gtile,
                                                 const int local_tile, RefSmem& sm,
                                                 const tilesort::Smem& ts)
 {
-    using S = RefShape<TW, TH>;
+    using S = RefShape<TW, TH, COLS>;
     constexpr int NC = S::NC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int first = __ldg(&a.ranges[2 * gtile]);
     const int last = __ldg(&a.ranges[2 * gtile + 1]);
     const int count = last - first;
     const int tx = local_tile % v.tiles_x, ty = local_tile / v.tiles_x;
-    const int px = tx * TW + (lane & 7) * NC, py0 = ty * TH + warp * 8 + (lane >> 3), py1 = py0 + 4;
+    const int px = tx * TW + (warp % S::WX) * 8 * NC + (lane & 7) * NC;
+    const int py0 = ty * TH + (warp / S::WX) * 8 + (lane >> 3), py1 = py0 + 4;
     const bool iny0 = py0 < v.height, iny1 = py1 < v.height;
     if (count <= 0) {
         // the reference clears the image and skips empty tiles (main.cpp:363);
@@ -426,10 +428,10 @@ __device__ __forceinline__ void raster_ref_tile(const RasterArgs& a, const ViewP
 // One CTA per tile of every view, in the raster order when there is one.
 // 640 threads per SM (96 registers): the FP32 pipe is busy with 20 warps, and
 // more of them only slow the heaviest tiles down (768 threads: raster +3 %).
-template <int TW, int TH>
-__global__ void __launch_bounds__(RefShape<TW, TH>::NT, 640 / RefShape<TW, TH>::NT) raster_ref_kernel(RasterArgs a)
+template <int TW, int TH, int COLS>
+__global__ void __launch_bounds__(RefShape<TW, TH, COLS>::NT, 640 / RefShape<TW, TH, COLS>::NT) raster_ref_kernel(RasterArgs a)
 {
-    using S = RefShape<TW, TH>;
+    using S = RefShape<TW, TH, COLS>;
     __shared__ RefSmem sm;
     __shared__ uint64_t s_k[S::CAP];
     __shared__ int32_t s_v[S::CAP];
@@ -447,7 +449,7 @@ __global__ void __launch_bounds__(RefShape<TW, TH>::NT, 640 / RefShape<TW, TH>::
     const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[a.tile_base + blockIdx.x]) : a.tile_base + blockIdx.x;
     const ViewParams& v = view_of_tile(a, gtile);
     stamp_start(a);
-    raster_ref_tile<TW, TH>(a, v, gtile, (int)(gtile - v.tile_offset), sm, ts);
+    raster_ref_tile<TW, TH, COLS>(a, v, gtile, (int)(gtile - v.tile_offset), sm, ts);
     stamp_end(a);
 }
 
@@ -494,9 +496,10 @@ __global__ void __launch_bounds__(TW * TH, 2048 / (TW * TH) * 5 / 8) raster_kern
 // 1280x720 views of 1M 0.99 -> 0.83 ms, of one 1080p view 0.195 -> 0.175 ms.
 // 640 threads per SM (96 registers): 768 with 80 registers spill in the sort
 // and take 13.2 ms, 896 and 1024 take 14.0 ms.
-template <int TW, int TH>
+template <int TW, int TH, int BLOCKS>
 struct RecShape {
-    static constexpr int BPW = TW / 8;              // 8x8 blocks per warp
+    static constexpr int BPW = BLOCKS;              // 8x8 blocks per warp, side by side
+    static constexpr int WX = TW / (8 * BPW);       // warps across a tile
     static constexpr int NT = TW * TH / (2 * BPW);  // threads: 2 BPW pixels each
     static constexpr int CAP = TW * TH / 2 * kFusedIpt;
 };
@@ -505,9 +508,9 @@ struct RecShape {
 // is sorted, in their place the tile's slots in blend order and every block's
 // survivors, double-buffered.
 constexpr int kRecStep = 32;  // entries a warp culls and stages at a time
-template <int TW, int TH>
+template <int TW, int TH, int BLOCKS>
 union RecSmem {
-    using S = RecShape<TW, TH>;
+    using S = RecShape<TW, TH, BLOCKS>;
     static constexpr int NB = TW * TH / 64;
     struct {
         uint64_t k[S::CAP];
@@ -528,10 +531,10 @@ union RecSmem {
 // One tile of the record raster.  Every thread of the CTA must call it (the
 // fused sort synchronises the CTA).  CHUNK (32 or 64) = the entries between
 // two tests of whether a block is done.
-template <int TW, int TH, int CHUNK>
-__device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64_t gtile, RecSmem<TW, TH>& sm)
+template <int TW, int TH, int CHUNK, int BLOCKS>
+__device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64_t gtile, RecSmem<TW, TH, BLOCKS>& sm)
 {
-    using S = RecShape<TW, TH>;
+    using S = RecShape<TW, TH, BLOCKS>;
     constexpr int BPW = S::BPW;
     constexpr int LPB = 32 / BPW;  // lanes per block
     constexpr int LX = 8 / BPW;    // lanes across a block
@@ -541,7 +544,8 @@ __device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64
     const int first = __ldg(&a.ranges[2 * gtile]);
     const int count = __ldg(&a.ranges[2 * gtile + 1]) - first;
     const int tx = local_tile % v.tiles_x, ty = local_tile / v.tiles_x;
-    const int wx0 = tx * TW, wy0 = ty * TH + warp * 8;  // the warp's blocks: (wx0 + 8 b, wy0)
+    // the warp's blocks: (wx0 + 8 b, wy0)
+    const int wx0 = tx * TW + (warp % S::WX) * 8 * BPW, wy0 = ty * TH + (warp / S::WX) * 8;
     const int half = lane / LPB, sub = lane % LPB;
     const int px = wx0 + 8 * half + (sub % LX) * BPW, py0 = wy0 + sub / LX, py1 = py0 + 4;
     const bool iny0 = py0 < v.height, iny1 = py1 < v.height;
@@ -711,26 +715,26 @@ __device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64
 }
 
 // One CTA per tile of [tile_base, tile_base + grid), in the raster order.
-template <int TW, int TH, int CHUNK>
-__global__ void __launch_bounds__(RecShape<TW, TH>::NT, 640 / RecShape<TW, TH>::NT) raster_rec_kernel(RasterArgs a)
+template <int TW, int TH, int CHUNK, int BLOCKS>
+__global__ void __launch_bounds__(RecShape<TW, TH, BLOCKS>::NT, 640 / RecShape<TW, TH, BLOCKS>::NT) raster_rec_kernel(RasterArgs a)
 {
-    __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH>)];
-    RecSmem<TW, TH>& sm = *reinterpret_cast<RecSmem<TW, TH>*>(smem);
+    __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH, BLOCKS>)];
+    RecSmem<TW, TH, BLOCKS>& sm = *reinterpret_cast<RecSmem<TW, TH, BLOCKS>*>(smem);
     const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[a.tile_base + blockIdx.x]) : a.tile_base + blockIdx.x;
     stamp_start(a);
-    raster_rec_tile<TW, TH, CHUNK>(a, gtile, sm);
+    raster_rec_tile<TW, TH, CHUNK, BLOCKS>(a, gtile, sm);
     stamp_end(a);
 }
 
 // Persistent CTAs (as many as fit on the SMs at once) that pull tiles from
 // an atomic queue over the raster order (heavy tiles first) until it runs
 // dry.
-template <int TW, int TH, int CHUNK>
-__global__ void __launch_bounds__(RecShape<TW, TH>::NT, 640 / RecShape<TW, TH>::NT)
+template <int TW, int TH, int CHUNK, int BLOCKS>
+__global__ void __launch_bounds__(RecShape<TW, TH, BLOCKS>::NT, 640 / RecShape<TW, TH, BLOCKS>::NT)
     raster_rec_persistent_kernel(RasterArgs a)
 {
-    __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH>)];
-    RecSmem<TW, TH>& sm = *reinterpret_cast<RecSmem<TW, TH>*>(smem);
+    __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH, BLOCKS>)];
+    RecSmem<TW, TH, BLOCKS>& sm = *reinterpret_cast<RecSmem<TW, TH, BLOCKS>*>(smem);
     __shared__ int64_t s_tile;
     stamp_start(a);
     for (;;) {
@@ -741,44 +745,61 @@ __global__ void __launch_bounds__(RecShape<TW, TH>::NT, 640 / RecShape<TW, TH>::
         __syncthreads();
         const int64_t gtile = s_tile;
         if (gtile < 0) break;
-        raster_rec_tile<TW, TH, CHUNK>(a, gtile, sm);
+        raster_rec_tile<TW, TH, CHUNK, BLOCKS>(a, gtile, sm);
         __syncthreads();  // s_tile and the sort's shared memory are reused
     }
     stamp_end(a);
 }
 
-template <int TW, int TH, int CHUNK>
+template <int TW, int TH, int CHUNK, int BLOCKS>
 static void launch_rec(const RasterArgs& a, bool persistent, int num_sms, cudaStream_t st)
 {
     if (a.num_tiles_total <= 0) return;
     if (!persistent) {
-        raster_rec_kernel<TW, TH, CHUNK><<<(unsigned)a.num_tiles_total, RecShape<TW, TH>::NT, 0, st>>>(a);
+        raster_rec_kernel<TW, TH, CHUNK, BLOCKS><<<(unsigned)a.num_tiles_total, RecShape<TW, TH, BLOCKS>::NT, 0, st>>>(a);
         return;
     }
     static int per_sm = 0;  // same on every B200; queried once
     if (per_sm == 0) {
         int x = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x, raster_rec_persistent_kernel<TW, TH, CHUNK>,
-                                                      RecShape<TW, TH>::NT, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x, raster_rec_persistent_kernel<TW, TH, CHUNK, BLOCKS>,
+                                                      RecShape<TW, TH, BLOCKS>::NT, 0);
         per_sm = std::max(x, 1);
     }
     const int64_t grid = std::min<int64_t>((int64_t)per_sm * num_sms, a.num_tiles_total);
-    raster_rec_persistent_kernel<TW, TH, CHUNK><<<(unsigned)grid, RecShape<TW, TH>::NT, 0, st>>>(a);
+    raster_rec_persistent_kernel<TW, TH, CHUNK, BLOCKS><<<(unsigned)grid, RecShape<TW, TH, BLOCKS>::NT, 0, st>>>(a);
+}
+
+// A launch of few tiles lasts as long as its longest ones, so it gives a tile
+// twice the warps, of half the pixels each; many tiles are a matter of
+// throughput, where the shared reads and terms of the wide lanes pay.  Raster,
+// twice the warps against wide lanes: 300 tiles 8 / 12 us (reference mode 12 /
+// 16), 1200 tiles 41 / 59 (88 / 116), 1900 tiles 38 / 49 (80 / 94), 2800 tiles
+// 62 / 63 (84 / 93); 4096 tiles (397 / 368), 8160 tiles 172 / 153.
+constexpr int kSmallTilesPerSm = 20;
+
+template <int TW, int TH, int WIDE>
+static void launch_width(const RasterArgs& a, int termination, int num_sms, cudaStream_t st)
+{
+    const unsigned tiles = (unsigned)a.num_tiles_total;
+    if (termination == 0)
+        raster_ref_kernel<TW, TH, WIDE><<<tiles, RefShape<TW, TH, WIDE>::NT, 0, st>>>(a);
+    else if (!a.rec)
+        raster_kernel<TW, TH><<<tiles, TW * TH, 0, st>>>(a);
+    else if (a.rec_chunk == 64)
+        launch_rec<TW, TH, 64, WIDE>(a, a.rec_persistent != 0, num_sms, st);
+    else
+        launch_rec<TW, TH, 32, WIDE>(a, a.rec_persistent != 0, num_sms, st);
 }
 
 template <int TW, int TH>
 static void launch_shape(const RasterArgs& a, int termination, int num_sms, cudaStream_t st)
 {
     if (a.num_tiles_total <= 0) return;
-    const unsigned tiles = (unsigned)a.num_tiles_total;
-    if (termination == 0)
-        raster_ref_kernel<TW, TH><<<tiles, RefShape<TW, TH>::NT, 0, st>>>(a);
-    else if (!a.rec)
-        raster_kernel<TW, TH><<<tiles, TW * TH, 0, st>>>(a);
-    else if (a.rec_chunk == 64)
-        launch_rec<TW, TH, 64>(a, a.rec_persistent != 0, num_sms, st);
+    if (a.num_tiles_total <= (int64_t)kSmallTilesPerSm * num_sms)
+        launch_width<TW, TH, 1>(a, termination, num_sms, st);
     else
-        launch_rec<TW, TH, 32>(a, a.rec_persistent != 0, num_sms, st);
+        launch_width<TW, TH, TW / 8>(a, termination, num_sms, st);
 }
 
 void launch_raster(const RasterArgs& a, int tile_w, int tile_h, int termination, int num_sms, cudaStream_t st)

@@ -19,7 +19,7 @@ def _lists(rng, tiles, n):
 
 
 @pytest.mark.parametrize("tile", [(16, 16), (16, 8), (8, 8)])
-@pytest.mark.parametrize("size", [(1, 1), (17, 9), (47, 33), (64, 48), (250, 131)])
+@pytest.mark.parametrize("size", [(1, 1), (17, 9), (47, 33), (64, 48), (250, 131), (1201, 651)])
 @pytest.mark.parametrize("wild", [False, True])
 def test_reference_raster(gs, O, tile, size, wild):
     import torch
@@ -58,14 +58,14 @@ def test_reference_raster(gs, O, tile, size, wild):
 
 @pytest.mark.parametrize("tile", [(16, 16), (16, 8), (8, 8)])
 @pytest.mark.parametrize("chunk", [32, 64])
-@pytest.mark.parametrize("n,size", [(1, (9, 5)), (40, (17, 16)), (700, (33, 47)), (9000, (50, 31))])
+@pytest.mark.parametrize("n,size", [(1, (9, 5)), (40, (17, 16)), (700, (33, 47)), (9000, (50, 31)), (9000, (1201, 651))])
 def test_record_raster(gs, O, tile, chunk, n, size):
     """Whole T_min frames whose blocks are cut by the image's edges, with one
     entry up to a few thousand per tile, against the oracle's raster of the
     frame's own lists and projected floats."""
     import torch
     W, H = size
-    sc = gs.scenes.uniform_scene(n, seed=n, log_scale_mu=-2.5)
+    sc = gs.scenes.uniform_scene(n, seed=n, log_scale_mu=-2.5 if W < 100 else -4.0)
     rc = gs.RenderConfig(tile_w=tile[0], tile_h=tile[1], raster_chunk=chunk)
     cam = gs.look_at((0.1, 0.2, 3.0), (0, 0, 0), (0, 1, 0), 50.0, W, H, 0.1, 100.0)
     ctx = gs.Context(0)
