@@ -786,6 +786,7 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ta.huge_count = &dc->huge_tiles;
     ta.fused_cap = fused_tile_capacity(cfg.tile_w, cfg.tile_h);
     ta.class_tiles = ctx->classes.as<unsigned int>();
+    ta.overlap = p.n > 0;
     const bool in_groups = p.host_copy && p.host_copy->groups > 1;
     ta.groups = in_groups ? p.host_copy->groups : 1;
     for (int g = 0; g < ta.groups; ++g) ta.group_tile[g] = in_groups ? p.host_copy->first_tile[g] : 0;
@@ -849,6 +850,7 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ra.fused_cap = fused_tile_capacity(cfg.tile_w, cfg.tile_h);
     ra.order = ea.order;
     ra.result = ctx->h_result;
+    ra.overlap = p.n > 0 && !in_groups;  // the groups' launches follow events and one another's streams
     ra.start_from = 1;
     ra.end_from = ra.num_tiles_total - kStampCtas;
     ra.rec_chunk = cfg.raster_chunk;

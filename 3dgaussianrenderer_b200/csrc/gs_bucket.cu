@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(kThreads) tile_scan_kernel(const __grid_consta
     __shared__ unsigned int s_class[kMaxRasterGroups * kOrderClasses];
     const int classes = a.groups * kOrderClasses;
     for (int k = threadIdx.x; k < classes; k += kThreads) s_class[k] = 0u;
+    frame_step_begin();
     if (threadIdx.x == 0) s_blk = (int64_t)atomicAdd(a.block_counter, 1ull);
     __syncthreads();
     const int64_t blk = s_blk;
@@ -177,7 +178,7 @@ void launch_tile_scan(const TileScanArgs& a, cudaStream_t st)
 {
     const int64_t blocks = (a.tiles + kTileScanItems - 1) / kTileScanItems;
     if (blocks <= 0) return;
-    tile_scan_kernel<<<(unsigned)blocks, kThreads, 0, st>>>(a);
+    launch_frame_step(tile_scan_kernel, (unsigned)blocks, kThreads, 0, st, a.overlap != 0, a);
 }
 
 // ---- 2. bucket emit -----------------------------------------------------------
@@ -204,6 +205,7 @@ __global__ void __launch_bounds__(kThreads, kEmitBlocksPerSm) emit_bucket_kernel
     constexpr int U = kEmitUnroll;
     constexpr int kBatch = kWarps * U;
     __shared__ unsigned long long s_next[2];
+    frame_step_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // straight into host memory: a copy at the frame's end would cost its
         // latency, and nothing after this kernel changes the words
@@ -299,7 +301,7 @@ void launch_emit_bucket(const BucketEmitArgs& a, int num_sms, cudaStream_t st)
     const int64_t work = std::max((a.chunk_capacity + batch - 1) / batch, (a.tiles + kThreads - 1) / kThreads);
     const int64_t blocks = std::min<int64_t>(work, (int64_t)num_sms * kEmitBlocksPerSm);
     if (blocks <= 0) return;
-    emit_bucket_kernel<<<(unsigned)blocks, kThreads, 0, st>>>(a);
+    launch_frame_step(emit_bucket_kernel, (unsigned)blocks, kThreads, 0, st, true, a);
 }
 
 // ---- 3. sort of the tiles too large for the raster CTAs -------------------------------
@@ -473,6 +475,7 @@ __global__ void __launch_bounds__(kBigThreads, kBigBlocksPerSm) tile_sort_big_ke
     sm.scan = s_scan;
     sm.red = s_red;
     sm.run = s_run;
+    frame_step_begin();
     const int nbig = (int)*a.big_count;
     for (int j = blockIdx.x; j < nbig; j += gridDim.x) {
         const int64_t t = a.big_list[j];
@@ -505,6 +508,7 @@ __global__ void __launch_bounds__(kHugeThreads, 1) tile_sort_huge_kernel(TileSor
     sm.scan = s_scan;
     sm.red = s_red;
     uint32_t* hist = reinterpret_cast<uint32_t*>(smem + kTileSortHugeKeys * 8);
+    frame_step_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0) stamp(a.result, kTimeSort);
     const int nhuge = (int)*a.huge_count;
     for (int j = blockIdx.x; j < nhuge; j += gridDim.x) {
@@ -533,8 +537,8 @@ void launch_tile_sort(const TileSortArgs& a, int num_sms, cudaStream_t st)
         cudaFuncSetAttribute(tile_sort_huge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, huge_smem);
     });
     if (a.tiles <= 0) return;
-    tile_sort_huge_kernel<<<(unsigned)num_sms, kHugeThreads, huge_smem, st>>>(a);
-    tile_sort_big_kernel<<<(unsigned)(kBigBlocksPerSm * num_sms), kBigThreads, big_smem, st>>>(a);
+    launch_frame_step(tile_sort_huge_kernel, (unsigned)num_sms, kHugeThreads, huge_smem, st, true, a);
+    launch_frame_step(tile_sort_big_kernel, (unsigned)(kBigBlocksPerSm * num_sms), kBigThreads, big_smem, st, true, a);
 }
 
 }  // namespace gs

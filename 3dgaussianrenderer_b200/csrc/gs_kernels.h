@@ -4,6 +4,7 @@
 #include "gs_common.cuh"
 
 #include <atomic>
+#include <utility>
 
 namespace gs {
 
@@ -80,6 +81,36 @@ __device__ __forceinline__ void stamp(FrameResult* r, const FrameTime k)
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     r->t[k] = t;
+}
+
+// The kernels of a bucket frame follow one another on the stream with
+// programmatic dependent launch: a kernel's blocks are scheduled while the one
+// before finishes its last ones, and wait in frame_step_begin until it has
+// completed and its writes are visible.  Every block of every such kernel waits,
+// so a kernel's completion implies that of all before it.  The first loads after
+// the wait whose address does not come from another such load are plain ones:
+// a read-only load (__ldg) may be moved up across the wait.
+__device__ __forceinline__ void frame_step_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... Params, class... Args>
+void launch_frame_step(void (*kernel)(Params...), const unsigned grid, const unsigned block, const size_t smem,
+                       cudaStream_t st, const bool overlap, Args&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);  // errors: the caller's cudaGetLastError
 }
 
 // Splats of more than kLargeCandidates candidate tiles are walked by
@@ -225,6 +256,7 @@ struct TileScanArgs {
     int32_t groups;
     int64_t group_tile[kMaxRasterGroups];  // first tile of each group
     unsigned int* class_tiles;       // [groups * kOrderClasses] tiles of each class; zero at launch
+    int32_t overlap;                 // 1: follows the large splats' kernel directly
 };
 
 // Per-tile sort of the buckets: each tile's keys are ordered by depth and,
@@ -330,6 +362,7 @@ struct RasterArgs {
     // a block is done (32 or 64), and a persistent grid over the atomic tile queue
     // (tile_counter, zero at launch) instead of one CTA per tile
     FrameResult* result;              // out: the raster's times; null: not wanted
+    int32_t overlap;                  // 1: follows the sort directly, see launch_frame_step
     int64_t start_from, end_from;     // CTAs before start_from stamp its start, those from end_from on its end
     int32_t rec_chunk;
     int32_t rec_persistent;

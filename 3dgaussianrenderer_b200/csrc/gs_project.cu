@@ -383,16 +383,16 @@ __global__ void __launch_bounds__(256) large_overlap_kernel(const __grid_constan
 {
     static_assert(kUnitCandidates == 1024, "one step of a unit per lane");
     const int lane = threadIdx.x & 31;
+    frame_step_begin();
     int64_t units = (int64_t)*a.unit_count;
     if (units > a.unit_capacity) units = a.unit_capacity;
     if (units == 0) return;
-    unsigned long long next = 0;
-    if (lane == 0) next = atomicAdd(a.unit_counter, 1ull);
-    for (;;) {
-        const int64_t k = (int64_t)__shfl_sync(kFull, next, 0);
-        if (k >= units) return;
+    // a warp's first unit is its own number, the next ones come from the counter
+    const int64_t warps = (int64_t)gridDim.x * 8;
+    int64_t k = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    for (unsigned long long next = 0; k < units; k = warps + (int64_t)__shfl_sync(kFull, next, 0)) {
         if (lane == 0) next = atomicAdd(a.unit_counter, 1ull);  // on its way while this unit is walked
-        const uint2 unit = __ldg(&a.units[k]);
+        const uint2 unit = a.units[k];
         const uint32_t slot = unit.x;
         const float2 centre = __ldg(&a.xy[slot]);
         const float4 el = __ldg(&a.ell[slot]);
@@ -590,6 +590,7 @@ __global__ void __launch_bounds__(256, (DEG >= 3 && !FAST) ? 3 : 4) frame_projec
     int gid = i;  // the Gaussian's caller index: equal depths are ordered by it
     if (BUCKET && a.orig) gid = __ldg(&a.orig[at]);
 
+    if (BUCKET) frame_step_begin();
     if (BUCKET && blockIdx.x == 0 && threadIdx.x == 0) stamp(a.result, kTimeStart);
     if (BUCKET && blockIdx.x == 0)
         for (int k = threadIdx.x; k < a.zero_count; k += 256) a.zero_words[k] = 0u;
@@ -951,7 +952,7 @@ void launch_frame_project(const FrameArgs& a, int deg, cudaStream_t st, bool buc
 
 void launch_large_overlaps(const FrameArgs& a, int num_sms, cudaStream_t st)
 {
-    large_overlap_kernel<<<(unsigned)(num_sms * 4), 256, 0, st>>>(a);
+    launch_frame_step(large_overlap_kernel, (unsigned)(num_sms * 4), 256, 0, st, true, a);
 }
 
 void launch_count_stage(const FrameArgs& a, cudaStream_t st)

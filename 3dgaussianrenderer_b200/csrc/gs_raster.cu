@@ -339,8 +339,8 @@ __device__ __forceinline__ void raster_ref_tile(const RasterArgs& a, const ViewP
     using S = RefShape<TW, TH, COLS>;
     constexpr int NC = S::NC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int first = __ldg(&a.ranges[2 * gtile]);
-    const int last = __ldg(&a.ranges[2 * gtile + 1]);
+    const int first = a.ranges[2 * gtile];
+    const int last = a.ranges[2 * gtile + 1];
     const int count = last - first;
     const int tx = local_tile % v.tiles_x, ty = local_tile / v.tiles_x;
     const int px = tx * TW + (warp % S::WX) * 8 * NC + (lane & 7) * NC;
@@ -446,7 +446,8 @@ __global__ void __launch_bounds__(RefShape<TW, TH, COLS>::NT, 640 / RefShape<TW,
     ts.scan = s_scan;
     ts.red = s_red;
     ts.run = nullptr;
-    const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[a.tile_base + blockIdx.x]) : a.tile_base + blockIdx.x;
+    frame_step_begin();
+    const int64_t gtile = a.order ? (int64_t)a.order[a.tile_base + blockIdx.x] : a.tile_base + blockIdx.x;
     const ViewParams& v = view_of_tile(a, gtile);
     stamp_start(a);
     raster_ref_tile<TW, TH, COLS>(a, v, gtile, (int)(gtile - v.tile_offset), sm, ts);
@@ -541,8 +542,8 @@ __device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const ViewParams& v = view_of_tile(a, gtile);
     const int local_tile = (int)(gtile - v.tile_offset);
-    const int first = __ldg(&a.ranges[2 * gtile]);
-    const int count = __ldg(&a.ranges[2 * gtile + 1]) - first;
+    const int first = a.ranges[2 * gtile];
+    const int count = a.ranges[2 * gtile + 1] - first;
     const int tx = local_tile % v.tiles_x, ty = local_tile / v.tiles_x;
     // the warp's blocks: (wx0 + 8 b, wy0)
     const int wx0 = tx * TW + (warp % S::WX) * 8 * BPW, wy0 = ty * TH + (warp / S::WX) * 8;
@@ -720,7 +721,8 @@ __global__ void __launch_bounds__(RecShape<TW, TH, BLOCKS>::NT, 640 / RecShape<T
 {
     __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH, BLOCKS>)];
     RecSmem<TW, TH, BLOCKS>& sm = *reinterpret_cast<RecSmem<TW, TH, BLOCKS>*>(smem);
-    const int64_t gtile = a.order ? (int64_t)__ldg(&a.order[a.tile_base + blockIdx.x]) : a.tile_base + blockIdx.x;
+    frame_step_begin();
+    const int64_t gtile = a.order ? (int64_t)a.order[a.tile_base + blockIdx.x] : a.tile_base + blockIdx.x;
     stamp_start(a);
     raster_rec_tile<TW, TH, CHUNK, BLOCKS>(a, gtile, sm);
     stamp_end(a);
@@ -736,11 +738,12 @@ __global__ void __launch_bounds__(RecShape<TW, TH, BLOCKS>::NT, 640 / RecShape<T
     __shared__ __align__(16) unsigned char smem[sizeof(RecSmem<TW, TH, BLOCKS>)];
     RecSmem<TW, TH, BLOCKS>& sm = *reinterpret_cast<RecSmem<TW, TH, BLOCKS>*>(smem);
     __shared__ int64_t s_tile;
+    frame_step_begin();
     stamp_start(a);
     for (;;) {
         if (threadIdx.x == 0) {
             const int64_t k = (int64_t)atomicAdd(a.tile_counter, 1ull);
-            s_tile = k < a.num_tiles_total ? (a.order ? (int64_t)__ldg(&a.order[a.tile_base + k]) : a.tile_base + k) : -1;
+            s_tile = k < a.num_tiles_total ? (a.order ? (int64_t)a.order[a.tile_base + k] : a.tile_base + k) : -1;
         }
         __syncthreads();
         const int64_t gtile = s_tile;
@@ -756,7 +759,8 @@ static void launch_rec(const RasterArgs& a, bool persistent, int num_sms, cudaSt
 {
     if (a.num_tiles_total <= 0) return;
     if (!persistent) {
-        raster_rec_kernel<TW, TH, CHUNK, BLOCKS><<<(unsigned)a.num_tiles_total, RecShape<TW, TH, BLOCKS>::NT, 0, st>>>(a);
+        launch_frame_step(raster_rec_kernel<TW, TH, CHUNK, BLOCKS>, (unsigned)a.num_tiles_total,
+                          RecShape<TW, TH, BLOCKS>::NT, 0, st, a.overlap != 0, a);
         return;
     }
     static int per_sm = 0;  // same on every B200; queried once
@@ -767,7 +771,8 @@ static void launch_rec(const RasterArgs& a, bool persistent, int num_sms, cudaSt
         per_sm = std::max(x, 1);
     }
     const int64_t grid = std::min<int64_t>((int64_t)per_sm * num_sms, a.num_tiles_total);
-    raster_rec_persistent_kernel<TW, TH, CHUNK, BLOCKS><<<(unsigned)grid, RecShape<TW, TH, BLOCKS>::NT, 0, st>>>(a);
+    launch_frame_step(raster_rec_persistent_kernel<TW, TH, CHUNK, BLOCKS>, (unsigned)grid, RecShape<TW, TH, BLOCKS>::NT, 0, st,
+                      a.overlap != 0, a);
 }
 
 // A launch of few tiles lasts as long as its longest ones, so it gives a tile
@@ -783,7 +788,7 @@ static void launch_width(const RasterArgs& a, int termination, int num_sms, cuda
 {
     const unsigned tiles = (unsigned)a.num_tiles_total;
     if (termination == 0)
-        raster_ref_kernel<TW, TH, WIDE><<<tiles, RefShape<TW, TH, WIDE>::NT, 0, st>>>(a);
+        launch_frame_step(raster_ref_kernel<TW, TH, WIDE>, tiles, RefShape<TW, TH, WIDE>::NT, 0, st, a.overlap != 0, a);
     else if (!a.rec)
         raster_kernel<TW, TH><<<tiles, TW * TH, 0, st>>>(a);
     else if (a.rec_chunk == 64)
