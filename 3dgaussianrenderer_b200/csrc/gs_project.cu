@@ -167,7 +167,7 @@ __device__ __forceinline__ int warp_count_hits(const Ell& e, const int4 r, const
     const WarpCands w = warp_scan_cands(cand - (pre ? 1 : 0));
     int hits = pre ? 1 : 0;
     mask = (pre && cand <= 32) ? (1u << c0) : 0u;
-    bool undecided = false;
+    unsigned undecided = 0;  // this lane's candidates too close to call: bit s of step s, bit 31 of all from 31
     for (int base = 0; base < w.total; base += 32) {
         const int c = base + lane;
         const int o = owner_of(w.incl, c);
@@ -179,12 +179,14 @@ __device__ __forceinline__ int warp_count_hits(const Ell& e, const int4 r, const
         int st = 0;
         int tile = 0;
         if (c < w.total) st = candidate_state(oe, orr, walk_candidate(c - oexcl, oc0), v, tile);
-        undecided |= st < 0;
+        undecided |= st < 0 ? 1u << min(base >> 5, 31) : 0u;
         add_hits(__ballot_sync(kFull, st > 0), w, base, cand, c0, hits, mask);
     }
-    if (__any_sync(kFull, undecided)) {
-        // rare: the candidates too close to call, in IEEE arithmetic
+    undecided = __reduce_or_sync(kFull, undecided);
+    if (undecided) {
+        // the steps that hold a candidate too close to call, in IEEE arithmetic
         for (int base = 0; base < w.total; base += 32) {
+            if (!((undecided >> min(base >> 5, 31)) & 1u)) continue;
             const int c = base + lane;
             const int o = owner_of(w.incl, c);
             Ell oe;
@@ -315,13 +317,13 @@ __device__ __forceinline__ unsigned run_walk(const Ell& e, const int2 pr, const 
     const int steps = (k.total + 31) >> 5;
     unsigned reached = k.preb;
     uint32_t chunk = 0;  // of the pending overlaps
-    bool undecided = false;
+    unsigned undecided = 0;  // this lane's candidates too close to call: bit s of step s
     mine = 0;
     for (int s = 0; s < steps; ++s) {
         int o, tile;
         Ell oe;
         const int st = walk_step(e, pr, k, s, v, oe, o, tile);
-        undecided |= st < 0;
+        undecided |= st < 0 ? 1u << s : 0u;
         const bool hit = st > 0;
         const unsigned bal = __ballot_sync(kFull, hit);
         if (lane == s) mine = bal;
@@ -332,16 +334,20 @@ __device__ __forceinline__ unsigned run_walk(const Ell& e, const int2 pr, const 
         if (s > 0 || k.preb) write_pending(a, x, chunk++);
         x = {(toff + (uint32_t)tile) | ((uint32_t)o << kOverlapTileBits), rank, lane, 0, hit};
     }
-    if (__any_sync(kFull, undecided)) {
-        // rare: the candidates too close to call, in IEEE arithmetic
+    undecided = __reduce_or_sync(kFull, undecided);
+    if (undecided) {
+        // the steps that hold a candidate too close to call, in IEEE arithmetic.
+        // Walking all steps again doubled the time of such a warp, and a frame
+        // of one wave waits for its longest (to the emission, 100k Gaussians 56
+        // -> 47 us; 64 views of 3M 6.28 -> 5.89 ms).
         write_pending(a, x, chunk);
         x.has = false;
         const uint32_t chunk0 = chunk - (uint32_t)(steps - 1);
-        for (int s = 0; s < steps; ++s) {
+        for (; undecided; undecided &= undecided - 1) {
+            const int s = __ffs(undecided) - 1;
             int o, tile;
             Ell oe;
             bool hit = walk_step(e, pr, k, s, v, oe, o, tile) < 0;
-            if (!__any_sync(kFull, hit)) continue;
             if (hit) hit = candidate_hit_ieee(oe, tile, v);
             const unsigned bal = __ballot_sync(kFull, hit);
             if (lane == s) mine |= bal;

@@ -54,3 +54,29 @@ def test_tile_lists(gs, O, n, mu, sigma, mode, views):
         assert np.array_equal((color.cpu().numpy() != 0).any(1), reached)
     scene.close()
     ctx.close()
+
+
+# Needles of a minor extent far below a pixel: many candidates are too close to
+# call and settled in the second walk, in early steps of a warp's walk and, at
+# the longer extents, in steps from 31 on.
+@pytest.mark.parametrize("n,length", [(1, 400.0), (33, 30.0), (33, 900.0), (5000, 12.0), (2000, 250.0)])
+@pytest.mark.parametrize("width", [1e-3, 0.2])
+def test_stage_build_of_needles(gs, O, n, length, width):
+    import torch
+    rng = np.random.default_rng(n + int(length))
+    w, h = 720, 500
+    cam = gs.look_at((0, 0, 2), (0, 0, 0), (0, 1, 0), 60.0, w, h, 0.1, 100.0)
+    rc = gs.RenderConfig.reference()
+    xy = (rng.random((n, 2)) * (w, h)).astype(np.float32)
+    a = rng.random(n) * np.pi
+    ell = np.stack([np.cos(a), np.sin(a), length * (0.5 + rng.random(n)), np.full(n, width)], 1).astype(np.float32)
+    z = rng.random(n).astype(np.float32)
+    keys, vals = O.build(xy, ell, z, cam, rc)
+    ctx = gs.Context(0)
+    dev = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()  # noqa: E731
+    cap = max(len(keys), 1)
+    dk, dv = torch.zeros(cap, dtype=torch.int64, device="cuda"), torch.zeros(cap, dtype=torch.int32, device="cuda")
+    K = gs.stage_build(ctx, n, dev(xy), dev(z), dev(ell), cam, rc, dk, dv, cap)
+    assert K == len(keys)
+    assert np.array_equal(dk.cpu().numpy()[:K].view(np.uint64), keys) and np.array_equal(dv.cpu().numpy()[:K], vals)
+    ctx.close()
