@@ -78,9 +78,14 @@ __device__ __forceinline__ uint64_t varying_bits_block(uint64_t or_v, uint64_t a
 // Raster order: tiles go to the rasteriser by falling key count, in classes of
 // half an octave (class 0 the heaviest), so that the longest CTAs start first
 // and the last wave is made of the shortest.
+//
+// Tiles of fewer than 16 keys, the empty ones among them, are one class: with
+// the empty tiles in a class of their own, at the end, a frame of many had a
+// phase of nothing but CTA launches (raster of 17 views of 14k Gaussians in
+// 384000 tiles of 8x8, half of them empty: 449 against 397 us).
 __device__ __forceinline__ int order_class(const uint32_t count)
 {
-    if (count == 0) return kOrderClasses - 1;
+    if (count < 16) return kOrderClasses - 9;
     const int l = 31 - __clz((int)count);
     const int half = 2 * l + (l > 0 ? (int)((count >> (l - 1)) & 1u) : 0);
     return kOrderClasses - 2 - min(half, kOrderClasses - 2);
