@@ -303,7 +303,7 @@ class RenderConfig:
     sort_variant: int = 0
     views_per_block: int = 0
     graph: int = 1
-    raster_chunk: int = 0       # T_min raster: Gaussians per shared-memory batch (0 = 32, or 64)
+    raster_chunk: int = 0       # T_min raster: entries between two done tests (0 = 32, or 64)
     raster_persistent: int = 0  # T_min raster: persistent CTAs over the atomic tile queue
     sort_bits: int = 0          # per-tile sort: radix-sorted top depth bits (0 = 16, 8..32)
 

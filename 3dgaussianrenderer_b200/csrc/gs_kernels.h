@@ -86,7 +86,8 @@ __device__ __forceinline__ void stamp(FrameResult* r, const FrameTime k)
 // The kernels of a bucket frame follow one another on the stream with
 // programmatic dependent launch: a kernel's blocks are scheduled while the one
 // before finishes its last ones, and wait in frame_step_begin until it has
-// completed and its writes are visible.  Every block of every such kernel waits,
+// completed and its writes are visible (single view of 100k Gaussians 159 ->
+// 152 us, of 1M 305 -> 295 us; batches unchanged).  Every block of every such kernel waits,
 // so a kernel's completion implies that of all before it.  The first loads after
 // the wait whose address does not come from another such load are plain ones:
 // a read-only load (__ldg) may be moved up across the wait.

@@ -76,8 +76,8 @@ typedef struct gs_render_cfg {
     int32_t views_per_block; /* views the fused projection handles per block (0 = 16) */
     int32_t graph;         /* 1 (default): a frame whose scene, options and views' sizes and outputs repeat
                               is captured once into a CUDA graph and replayed; 0: plain stream launches */
-    int32_t raster_chunk;  /* GS_TERM_TMIN raster: Gaussians each warp culls and stages in shared memory per
-                              step, 32 or 64 (0 = 32) */
+    int32_t raster_chunk;  /* GS_TERM_TMIN raster: a block of pixels tests whether it is done every so many
+                              entries of its tile, 32 or 64 (0 = 32) */
     int32_t raster_persistent; /* GS_TERM_TMIN raster: 1 = persistent CTAs pulling tiles (heavy first) from an
                               atomic queue; 0 (default) = one CTA per tile */
     int32_t sort_bits;     /* per-tile depth sort of GS_ORDER_BUCKETS frames inside the raster CTA: the top
@@ -106,7 +106,8 @@ typedef struct gs_stats {
     int64_t num_tiles;
     int64_t kernel_launches; /* gs_b200 kernels launched for the frame */
     int32_t graph_replay;    /* 1: the frame ran as a replay of a captured CUDA graph */
-    int32_t attempts;        /* launches of the frame: 2 when the tile list outgrew its buffers and was redone;
+    int32_t attempts;        /* launches of the frame: 2 when the tile list outgrew its buffers and was redone (3 when
+                                the units of its large splats did not fit either);
                                 a batch whose tile lists need 2^31 entries or more (or whose views x Gaussians
                                 reach 2^31) renders as frames over halves of its views, with the same images:
                                 the halves' stats add up and attempts counts the frame that found it too big */
@@ -209,8 +210,8 @@ typedef struct gs_tune_result {
  *   sort_variant 0..3               onesweep ordering;
  *   sort_bits 8 / 16 / 24 / 32      bucket ordering (the per-tile sort's
  *                                   radix width);
- *   raster_chunk 32 / 64            GS_TERM_TMIN (Gaussians per
- *                                   shared-memory batch of the raster);
+ *   raster_chunk 32 / 64            GS_TERM_TMIN (entries between two tests
+ *                                   of whether a block is done);
  *   raster_persistent 0 / 1         GS_TERM_TMIN.
  * The sorts are exact, so sort knobs never change an image; raster_chunk
  * moves where a warp notices that its pixels are done, which changes colours
