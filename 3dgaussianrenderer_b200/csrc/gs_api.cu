@@ -162,7 +162,7 @@ constexpr size_t kHostGroupBytes = 2u << 20;
 // The raster's last CTAs that stamp its end: enough that the last one to finish
 // is among them (the order puts the long ones first), few enough that their
 // writes to host memory do not hold up the images' copies.
-constexpr int64_t kStampCtas = 2048;
+constexpr int32_t kStampCtas = 2048;
 
 // Host read-back overlapped with the frame (bucket frames): the raster runs in
 // groups of tile rows, one after the other in image order, each group's end is
@@ -858,8 +858,8 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ra.result = ctx->h_result;
     // the groups' launches follow events and one another's streams
     ra.overlap = p.n > 0 && !in_groups && p.tiles_total <= kOverlapTiles;
-    ra.start_from = 1;
-    ra.end_from = ra.num_tiles_total - kStampCtas;
+    ra.stamp_start = 1;
+    ra.end_ctas = kStampCtas;
     ra.rec_chunk = cfg.raster_chunk;
     ra.rec_persistent = cfg.raster_persistent;
     ra.sort_prefix_bits = cfg.sort_bits;
@@ -879,8 +879,8 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
             RasterArgs rg = ra;
             rg.tile_base = hc.first_tile[g];
             rg.num_tiles_total = hc.first_tile[g + 1] - hc.first_tile[g];
-            rg.start_from = g == 0 ? 1 : 0;
-            rg.end_from = g + 2 >= hc.groups ? rg.num_tiles_total - kStampCtas : rg.num_tiles_total;
+            rg.stamp_start = g == 0 ? 1 : 0;
+            rg.end_ctas = g + 2 >= hc.groups ? kStampCtas : 0;
             // a persistent group launch starts its own queue from zero
             if (rg.rec_persistent) GS_CUDA(cudaMemsetAsync(&dc->raster_tile, 0, sizeof(unsigned long long), gst));
             launch_raster(rg, cfg.tile_w, cfg.tile_h, cfg.termination, ctx->num_sms, gst);
@@ -1018,6 +1018,7 @@ int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, 
         ++attempts;
         ctx->h_init->epoch_scan = take_epochs(ctx->epoch_scan, 1, ctx->scan_status, st);
         ctx->h_init->epoch_sort = 0;
+        std::fill(ctx->h_result->t, ctx->h_result->t + kFrameTimes, 0ull);  // no older frame's time stands in
         // the second call with the same key is captured; a redone frame is not
         const bool use_graph = g && !g->failed && g->seen >= 2 && attempts == 1 && !ctx->tile_count_dirty;
         if (use_graph && !g->exec && !capture_frame(ctx, scene, cfg, p, *g)) g->failed = 1;

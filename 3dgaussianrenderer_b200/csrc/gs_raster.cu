@@ -213,14 +213,16 @@ __device__ __forceinline__ int slot_at(const RasterArgs& a, const uint64_t* sk, 
 }
 
 // The raster's times: its first CTA the start, every warp of the last CTAs the
-// end (the last writer stays).
+// end (the last writer stays).  Persistent CTAs end in any order, so all of
+// them stamp.
 __device__ __forceinline__ void stamp_start(const RasterArgs& a)
 {
-    if (a.result && blockIdx.x < a.start_from && threadIdx.x == 0) stamp(a.result, kTimeRaster);
+    if (a.result && a.stamp_start && blockIdx.x == 0 && threadIdx.x == 0) stamp(a.result, kTimeRaster);
 }
-__device__ __forceinline__ void stamp_end(const RasterArgs& a)
+__device__ __forceinline__ void stamp_end(const RasterArgs& a, const bool persistent = false)
 {
-    if (a.result && blockIdx.x >= a.end_from && (threadIdx.x & 31) == 0) stamp(a.result, kTimeEnd);
+    if (!a.result || !a.end_ctas || (threadIdx.x & 31) != 0) return;
+    if (persistent || blockIdx.x + (unsigned)a.end_ctas >= gridDim.x) stamp(a.result, kTimeEnd);
 }
 
 // The view a global tile belongs to: binary search over the views' first tiles.
@@ -756,7 +758,7 @@ __global__ void __launch_bounds__(RecShape<TW, TH, BLOCKS>::NT, RecShape<TW, TH,
         raster_rec_tile<TW, TH, CHUNK, BLOCKS>(a, gtile, sm);
         __syncthreads();  // s_tile and the sort's shared memory are reused
     }
-    stamp_end(a);
+    stamp_end(a, true);
 }
 
 template <int TW, int TH, int CHUNK, int BLOCKS>
