@@ -159,9 +159,9 @@ constexpr int kHostChunkViews = 16;
 // takes 36 us at 55 GB/s, several times its launch and its group's.
 constexpr size_t kHostGroupBytes = 2u << 20;
 
-// The raster's last CTAs that stamp its end: enough that the last one to finish
-// is among them (the order puts the long ones first), few enough that their
-// writes to host memory do not hold up the images' copies.
+// The raster's last CTAs that stamp its end, with the long tiles (stamp_end):
+// enough that a short tile among the others ends before them, few enough that
+// their writes to host memory do not hold up the images' copies.
 constexpr int32_t kStampCtas = 2048;
 
 // Host read-back overlapped with the frame (bucket frames): the raster runs in

@@ -365,7 +365,7 @@ struct RasterArgs {
     FrameResult* result;              // out: the raster's times; null: not wanted
     int32_t overlap;                  // 1: follows the sort directly, see launch_frame_step
     int32_t stamp_start;              // 1: the first CTA stamps the raster's start
-    int32_t end_ctas;                 // the last so many CTAs stamp its end (persistent: all of them); 0: none
+    int32_t end_ctas;                 // the last so many CTAs stamp its end (and long tiles, stamp_end); 0: none
     int32_t rec_chunk;
     int32_t rec_persistent;
     int32_t sort_prefix_bits;         // depth bits the fused tile sort radix-sorts (8..32; 0 = 16)

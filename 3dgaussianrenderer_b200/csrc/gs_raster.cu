@@ -212,17 +212,22 @@ __device__ __forceinline__ int slot_at(const RasterArgs& a, const uint64_t* sk, 
     return sk ? (int)(uint32_t)sk[idx] : __ldg(&a.values[first + idx]);
 }
 
-// The raster's times: its first CTA the start, every warp of the last CTAs the
-// end (the last writer stays).  Persistent CTAs end in any order, so all of
-// them stamp.
+// The raster's times: its first CTA stamps the start.  The end is stamped by
+// every warp of the last CTAs and of each tile of kStampKeys entries or more
+// (the last writer stays): a tile that is drawn early, but is long, may end
+// after all others.  A shorter one among the earlier CTAs takes 10 us or so, by
+// which the end may be early at the most.  Stamps of all tiles would cost a
+// frame whose images stream to the host 0.4 ms (24 views), and a short tile a
+// good part of its own time.  Persistent CTAs end in any order: all of them stamp.
+constexpr int kStampKeys = 512;
 __device__ __forceinline__ void stamp_start(const RasterArgs& a)
 {
     if (a.result && a.stamp_start && blockIdx.x == 0 && threadIdx.x == 0) stamp(a.result, kTimeRaster);
 }
-__device__ __forceinline__ void stamp_end(const RasterArgs& a, const bool persistent = false)
+__device__ __forceinline__ void stamp_end(const RasterArgs& a, const int count)
 {
     if (!a.result || !a.end_ctas || (threadIdx.x & 31) != 0) return;
-    if (persistent || blockIdx.x + (unsigned)a.end_ctas >= gridDim.x) stamp(a.result, kTimeEnd);
+    if (count >= kStampKeys || blockIdx.x + (unsigned)a.end_ctas >= gridDim.x) stamp(a.result, kTimeEnd);
 }
 
 // The view a global tile belongs to: binary search over the views' first tiles.
@@ -333,10 +338,11 @@ __device__ __forceinline__ bool wild_entry(const RefSmem& sm, const int j)
              fabsf(k.z) < 1e30f);
 }
 
+// One tile; returns its entries.
 template <int TW, int TH, int COLS>
-__device__ __forceinline__ void raster_ref_tile(const RasterArgs& a, const ViewParams& v, const int64_t gtile,
-                                                const int local_tile, RefSmem& sm,
-                                                const tilesort::Smem& ts)
+__device__ __forceinline__ int raster_ref_tile(const RasterArgs& a, const ViewParams& v, const int64_t gtile,
+                                               const int local_tile, RefSmem& sm,
+                                               const tilesort::Smem& ts)
 {
     using S = RefShape<TW, TH, COLS>;
     constexpr int NC = S::NC;
@@ -359,7 +365,7 @@ __device__ __forceinline__ void raster_ref_tile(const RasterArgs& a, const ViewP
                 if (iny1) v.out[(int64_t)py1 * v.width + px + i] = make_uchar4(0, 0, 0, 0);
             }
         }
-        return;
+        return 0;
     }
     const uint64_t* sk = fused_sort<S::NT, S::CAP>(a, first, count, ts);
     // pixel corner sample, gaussian_render.cu:701-704
@@ -425,6 +431,7 @@ __device__ __forceinline__ void raster_ref_tile(const RasterArgs& a, const ViewP
         if (iny0) store_pixel(v, px + i, py0, r0, g0, b0);
         if (iny1) store_pixel(v, px + i, py1, r1, g1, b1);
     }
+    return count;
 }
 
 // One CTA per tile of every view, in the raster order when there is one.
@@ -452,8 +459,7 @@ __global__ void __launch_bounds__(RefShape<TW, TH, COLS>::NT, 640 / RefShape<TW,
     const int64_t gtile = a.order ? (int64_t)a.order[a.tile_base + blockIdx.x] : a.tile_base + blockIdx.x;
     const ViewParams& v = view_of_tile(a, gtile);
     stamp_start(a);
-    raster_ref_tile<TW, TH, COLS>(a, v, gtile, (int)(gtile - v.tile_offset), sm, ts);
-    stamp_end(a);
+    stamp_end(a, raster_ref_tile<TW, TH, COLS>(a, v, gtile, (int)(gtile - v.tile_offset), sm, ts));
 }
 
 template <int TW, int TH>
@@ -537,9 +543,9 @@ union RecSmem {
 
 // One tile of the record raster.  Every thread of the CTA must call it (the
 // fused sort synchronises the CTA).  CHUNK (32 or 64) = the entries between
-// two tests of whether a block is done.
+// two tests of whether a block is done.  Returns the tile's entries.
 template <int TW, int TH, int CHUNK, int BLOCKS>
-__device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64_t gtile, RecSmem<TW, TH, BLOCKS>& sm)
+__device__ __forceinline__ int raster_rec_tile(const RasterArgs& a, const int64_t gtile, RecSmem<TW, TH, BLOCKS>& sm)
 {
     using S = RecShape<TW, TH, BLOCKS>;
     constexpr int BPW = S::BPW;
@@ -566,7 +572,7 @@ __device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64
                 if (iny1) v.out[(int64_t)py1 * v.width + px + c] = make_uchar4(0, 0, 0, 0);
             }
         }
-        return;
+        return 0;
     }
     const bool sorted_here = a.keys && count <= a.fused_cap;
     if (sorted_here) {
@@ -720,6 +726,7 @@ __device__ __forceinline__ void raster_rec_tile(const RasterArgs& a, const int64
         if (iny0) store_pixel(v, px + c, py0, r0, g0, b0);
         if (iny1) store_pixel(v, px + c, py1, r1, g1, b1);
     }
+    return count;
 }
 
 // One CTA per tile of [tile_base, tile_base + grid), in the raster order.
@@ -731,8 +738,7 @@ __global__ void __launch_bounds__(RecShape<TW, TH, BLOCKS>::NT, RecShape<TW, TH,
     if (a.overlap) frame_step_begin();
     const int64_t gtile = a.order ? (int64_t)a.order[a.tile_base + blockIdx.x] : a.tile_base + blockIdx.x;
     stamp_start(a);
-    raster_rec_tile<TW, TH, CHUNK, BLOCKS>(a, gtile, sm);
-    stamp_end(a);
+    stamp_end(a, raster_rec_tile<TW, TH, CHUNK, BLOCKS>(a, gtile, sm));
 }
 
 // Persistent CTAs (as many as fit on the SMs at once) that pull tiles from
@@ -758,7 +764,7 @@ __global__ void __launch_bounds__(RecShape<TW, TH, BLOCKS>::NT, RecShape<TW, TH,
         raster_rec_tile<TW, TH, CHUNK, BLOCKS>(a, gtile, sm);
         __syncthreads();  // s_tile and the sort's shared memory are reused
     }
-    stamp_end(a, true);
+    stamp_end(a, kStampKeys);
 }
 
 template <int TW, int TH, int CHUNK, int BLOCKS>

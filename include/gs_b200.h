@@ -99,7 +99,10 @@ typedef struct gs_render_cfg {
 #define GS_ORDER_AUTO 2
 
 /* Per-stage device times of one frame, same fields as the reference's
- * RenderStats (core/types.h:26-33), plus the tile-list size. */
+ * RenderStats (core/types.h:26-33), plus the tile-list size.  Bucket frames
+ * take them from the device's clock: the raster's end is that of its last CTAs
+ * and of its tiles of 512 entries or more, which a shorter tile may outlast by
+ * about 10 us.  Onesweep frames time the stages with events. */
 typedef struct gs_stats {
     double sh_eval_ms, project_ms, build_tile_ms, sort_ms, raster_ms, total_ms;
     int64_t num_keys;
