@@ -164,6 +164,10 @@ constexpr size_t kHostGroupBytes = 2u << 20;
 // their writes to host memory do not hold up the images' copies.
 constexpr int32_t kStampCtas = 2048;
 
+// Chunks of the overlap list hold 20 to 23 keys of their 32 on the benchmark's
+// views, fewer where a warp's splats are mostly out of view.
+constexpr int64_t kKeysPerChunk = 16;
+
 // Host read-back overlapped with the frame (bucket frames): the raster runs in
 // groups of tile rows, one after the other in image order, each group's end is
 // marked by an event, and its part of the images is copied on `copy` after it.
@@ -264,6 +268,7 @@ struct gs_ctx {
     DevBuf tile_count, big_list;           // tile-bucket ordering: keys per tile, big tiles
     DevBuf overlaps, chunks;               // tile-bucket ordering: the frame's overlap list (BucketEmitArgs)
     int64_t chunk_capacity = 0;
+    int64_t chunk_keys = 0;                // key capacity that the overlap list was sized for
     DevBuf tile_order;                     // raster order of the tiles (heavy tiles first)
     DevBuf counters;                       // of the other paths
     DevBuf classes;                        // raster order: tiles of each class, and how many of them are placed
@@ -430,15 +435,19 @@ int ensure_key_buffers(gs_ctx* ctx, int64_t keys)
     return GS_OK;
 }
 
-// Grows the overlap list of tile-bucket frames to hold `chunks` chunks.
+// Grows the overlap list of tile-bucket frames to hold `chunks` chunks, and
+// notes that it is the one that goes with the present key list.
 int ensure_overlaps(gs_ctx* ctx, int64_t chunks)
 {
+    ctx->chunk_keys = ctx->key_capacity;
     if (chunks <= ctx->chunk_capacity && ctx->overlaps.p) return GS_OK;
     const size_t c = (size_t)std::max<int64_t>(chunks, 1);
     ctx->chunk_capacity = 0;
+    ctx->chunk_keys = 0;
     if (ctx->overlaps.ensure(sizeof(uint2) * 32 * c) || ctx->chunks.ensure(sizeof(uint4) * c))
         return fail(GS_ERR_OOM, "overlap list");
     ctx->chunk_capacity = (int64_t)std::min(ctx->overlaps.bytes / (sizeof(uint2) * 32), ctx->chunks.bytes / sizeof(uint4));
+    ctx->chunk_keys = ctx->key_capacity;
     return GS_OK;
 }
 
@@ -977,8 +986,12 @@ int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, 
         rc = ensure_key_buffers(ctx, std::max<int64_t>(p.items, 1 << 20));
         if (rc) return rc;
     }
-    // a first guess of three chunks per two warps and views; a frame that needs more is redone
-    rc = ensure_overlaps(ctx, std::max<int64_t>(p.items / 32 * 3 / 2, 1 << 15));
+    // The overlap list is sized from the key list, so that a frame whose keys fit
+    // is seldom redone for its chunks: one chunk per kKeysPerChunk keys, as long
+    // as no frame has shown how many they really hold; three per two warps and
+    // views at least.
+    const int64_t by_keys = ctx->chunk_keys < ctx->key_capacity ? ctx->key_capacity / kKeysPerChunk : 0;
+    rc = ensure_overlaps(ctx, std::max<int64_t>(by_keys, p.items / 32 * 3 / 2));
     if (rc) return rc;
 
     // the graph slot of this frame, if any
@@ -1060,8 +1073,10 @@ int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, 
         const int64_t need = std::max(K > ctx->key_capacity ? K + K / 4 : 0, (int64_t)ctx->h_result->units);
         rc = ensure_key_buffers(ctx, std::min<int64_t>(need, (1ll << 31) - 1));
         if (rc) return rc;
+        // both lists grow by the same quarter, whichever was short, so that the
+        // next frame that is redone is so for both
         const int64_t chunks = (int64_t)(ctx->h_result->slots >> 32);
-        rc = ensure_overlaps(ctx, chunks);
+        rc = ensure_overlaps(ctx, chunks + chunks / 4);
         if (rc) return rc;
     }
 
