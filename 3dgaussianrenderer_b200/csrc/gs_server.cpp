@@ -95,10 +95,14 @@ size_t frame_bytes_estimate(const SceneEntry& s, const std::vector<Request>& req
 {
     size_t px = 0;
     for (const Request& r : reqs) px += 4 * (size_t)r.cam.width * r.cam.height;
-    const double views = (double)reqs.size();
-    // per (view, Gaussian) splat buffers + tile lists (keys/values, double
-    // buffered) + images
-    return (size_t)(views * s.n * 76.0 + views * s.n * s.keys_per_gaussian * 24.0) + px;
+    // What a context comes to hold for such a frame: 88 bytes of splat buffers
+    // per (view, Gaussian), and per place of the key list two keys and two
+    // values and a 16th of a 272-byte chunk of the overlap list.  The key list
+    // has a place per item at least and is regrown with a quarter more than it
+    // needed; every allocation has a quarter of headroom.
+    const double items = (double)reqs.size() * (double)s.n;
+    const double keys = std::max(1.0, 1.25 * s.keys_per_gaussian) * items;
+    return (size_t)(1.25 * (items * 88.0 + keys * (24.0 + 272.0 / 16.0))) + px;
 }
 
 void worker_loop(gs_server* S, Worker* w)
