@@ -428,8 +428,11 @@ __device__ bool count_sort_tile(const uint64_t* __restrict__ keys, const int m, 
             }
             b1 = lo;
             cnt = start(b1) - s0;
-            if (cnt == 0) return true;  // one bin has more than cap keys (uniform: every thread reads the same)
-            __syncthreads();            // starts are read before the placement moves them
+            if (cnt == 0) {  // one bin has more than cap keys (uniform: every thread reads the same)
+                too_long = true;
+                break;
+            }
+            __syncthreads();  // starts are read before the placement moves them
         }
         auto place = [&](const uint64_t k) {
             const uint32_t d = (uint32_t)(k >> shift) & (kBins - 1);
