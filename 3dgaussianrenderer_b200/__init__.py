@@ -169,6 +169,7 @@ _sig("gs_stage_raster", _I, ctypes.POINTER(gs_camera), ctypes.POINTER(gs_render_
 _sig("gs_probe_frame", _I, _P, _P, ctypes.POINTER(gs_camera), _I32, ctypes.POINTER(gs_render_cfg), ctypes.POINTER(_P),
      ctypes.POINTER(gs_frame_probe), ctypes.POINTER(gs_stats), _P)
 _sig("gs_probe_tile_lists", _I, _P, _P, _I64, _P, _P, _I64, _P, _I64, ctypes.POINTER(_I64), ctypes.POINTER(_I32))
+_sig("gs_probe_density", _I, _I64, _P, _P, _P, _P, _P)
 _sig("gs_test_fail_allocations", None, _I32, _I32)
 _sig("gs_test_pending_allocation_failures", _I32)
 _sig("gs_test_bounded_wait", _I, _I32, _P)
@@ -543,6 +544,13 @@ def probe_sort_timed(ctx: Context, num_keys, bits, src_keys, src_values, d_keys,
                                   _ptr(d_values), _ptr(d_keys_alt), _ptr(d_values_alt), iterations,
                                   ctypes.byref(sel), ctypes.byref(ms)), "gs_probe_sort_timed")
     return int(sel.value), ms.value
+
+
+def probe_density(d_q, d_wild, d_tame, d_expf, stream=None):
+    """gs_probe_density: the reference-mode raster's density of every q, in its
+    two forms, and the reference's expression as CUDA evaluates it."""
+    check(lib.gs_probe_density(d_q.numel(), _ptr(d_q), _ptr(d_wild), _ptr(d_tame), _ptr(d_expf), _stream_ptr(stream)),
+          "gs_probe_density")
 
 
 def stage_ranges(num_keys, d_keys, tiles, d_ranges, stream=None):

@@ -2206,4 +2206,13 @@ int gs_probe_tile_lists(gs_ctx* ctx, int32_t* h_ranges, int64_t ranges_capacity,
     return GS_OK;
 }
 
+int gs_probe_density(int64_t n, const float* d_q, float* d_wild, float* d_tame, float* d_expf, void* stream)
+{
+    if (n < 0 || n >= (1ll << 31) || (n > 0 && (!d_q || !d_wild || !d_tame || !d_expf)))
+        return fail(GS_ERR_INVALID, "bad argument");
+    launch_density_probe(n, d_q, d_wild, d_tame, d_expf, (cudaStream_t)stream);
+    GS_CUDA(cudaGetLastError());
+    return GS_OK;
+}
+
 }  // extern "C"

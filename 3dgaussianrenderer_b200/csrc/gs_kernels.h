@@ -402,6 +402,7 @@ int sort_passes(int key_bits);
 
 void launch_ranges(const uint64_t* keys, int64_t num_items, const int64_t* d_num_items, int32_t* ranges,
                    cudaStream_t st);
+void launch_density_probe(int64_t n, const float* q, float* wild, float* tame, float* expf_form, cudaStream_t st);
 void launch_raster(const RasterArgs& a, int tile_w, int tile_h, int termination, int num_sms, cudaStream_t st);
 
 // Scene storage order (gs_scene.cu): 30-bit Morton codes of the centres over

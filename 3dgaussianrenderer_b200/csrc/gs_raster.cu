@@ -290,18 +290,26 @@ __device__ __forceinline__ float ex2_approx(const float x)
     return y;
 }
 
-// sat(exp(-q/2)) of the exponent p = -log2(e)/2 q: 2^p, clamped to 1 above
-// and with NaN as 0.  Where p cannot be NaN (WILD false) the clamp is taken on
-// p instead, which moves it from the FP32 pipe, the loop's bound, to the ALU:
-// 2^0 is exactly 1 and 2^p is at most 1 for p <= 0.
+// exp(-q/2) = 2^p with p = -(log2(e) / 2) q, one product and one ex2.  The
+// product and the constant leave p off by at most |p| (2^-24 + 2^-26) and ex2 is
+// good to 2^-22 of its value, so the density is within 2^-22 + 3.8e-8 |q| of
+// itself; a result below 2^-126, which changes no colour, is flushed to 0.
+// gs_probe_density evaluates this form beside the call of __expf that the
+// reference makes: on 16M values of q all results of 2^-126 and above are the
+// same bits.
+constexpr float kExponentOfQ = -0.72134752f;
+
+// sat(2^p): clamped to 1 above and with NaN as 0.  Where p cannot be NaN (WILD
+// false) the clamp is taken on p instead, which moves it from the FP32 pipe,
+// the loop's bound, to the ALU: 2^0 is exactly 1 and 2^p is at most 1 for
+// p <= 0.
 template <bool WILD>
 __device__ __forceinline__ float density_of(const float p)
 {
     return WILD ? __saturatef(ex2_approx(p)) : ex2_approx(fminf(p, 0.0f));
 }
 
-// One entry into the lane's pixels.  Halving q is exact, so the one product
-// with -log2(e)/2 rounds as __expf's product of -0.5 q with log2(e) does.
+// One entry into the lane's pixels.
 template <int NC, bool WILD>
 __device__ __forceinline__ void blend_ref(const float (&cx)[NC], const f2 cy, const RefSmem& sm, const int j,
                                           f2 (&R)[NC], f2 (&G)[NC], f2 (&B)[NC], f2 (&T)[NC])
@@ -317,7 +325,7 @@ __device__ __forceinline__ void blend_ref(const float (&cx)[NC], const f2 cy, co
     for (int i = 0; i < NC; ++i) {
         const float dx = __fsub_rn(cx[i], c.x);
         const f2 inner = f2_fma(f2_dup(__fmul_rn(k.x, dx)), f2_dup(dx), cdy2);
-        const f2 p = f2_mul(f2_fma(f2_dup(__fmul_rn(kb2, dx)), dy, inner), f2_dup(-0.72134752f));
+        const f2 p = f2_mul(f2_fma(f2_dup(__fmul_rn(kb2, dx)), dy, inner), f2_dup(kExponentOfQ));
         float p0, p1;
         f2_unpack(p, p0, p1);
         const f2 alpha = f2_mul(op2, f2_pack(density_of<WILD>(p0), density_of<WILD>(p1)));
@@ -818,6 +826,27 @@ static void launch_shape(const RasterArgs& a, int termination, int num_sms, cuda
         launch_width<TW, TH, 1>(a, termination, num_sms, st);
     else
         launch_width<TW, TH, TW / 8>(a, termination, num_sms, st);
+}
+
+// gs_probe_density: the reference raster's density, the form of batches that
+// may hold a NaN and the other one, and the reference's expression.
+__global__ void __launch_bounds__(256) density_probe_kernel(const int64_t n, const float* __restrict__ q,
+                                                            float* __restrict__ wild, float* __restrict__ tame,
+                                                            float* __restrict__ expf_form)
+{
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    float p, unused;
+    f2_unpack(f2_mul(f2_dup(q[i]), f2_dup(kExponentOfQ)), p, unused);
+    wild[i] = density_of<true>(p);
+    tame[i] = density_of<false>(p);
+    expf_form[i] = __saturatef(__expf(__fmul_rn(-0.5f, q[i])));
+}
+
+void launch_density_probe(const int64_t n, const float* q, float* wild, float* tame, float* expf_form, cudaStream_t st)
+{
+    if (n <= 0) return;
+    density_probe_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, q, wild, tame, expf_form);
 }
 
 void launch_raster(const RasterArgs& a, int tile_w, int tile_h, int termination, int num_sms, cudaStream_t st)

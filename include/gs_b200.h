@@ -438,6 +438,12 @@ GS_API int gs_probe_sort_timed(gs_ctx* ctx, int64_t num_keys, int32_t key_bits, 
                                int32_t* d_values_alt, int32_t iterations, int32_t* out_selector,
                                double* out_median_ms);
 
+/* The density sat(exp(-q / 2)) of n values q as the reference-mode raster
+ * evaluates it, in the form of batches whose exponents may be NaN (d_wild) and
+ * in the other one (d_tame), and as CUDA evaluates the reference's expression
+ * (core/gaussian_render.cu:727-737) (d_expf).  Device pointers, n floats each. */
+GS_API int gs_probe_density(int64_t n, const float* d_q, float* d_wild, float* d_tame, float* d_expf, void* stream);
+
 /* ---- failure-path test hooks -------------------------------------------- */
 /* No counterpart in the reference, which exits the process on any CUDA
  * error (core/cuda_error_check.h:2-11).  These let tests exercise the error
