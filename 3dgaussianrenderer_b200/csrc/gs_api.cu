@@ -120,12 +120,11 @@ struct Counters {
     unsigned long long slots;                      // frame kernel: (view, Gaussian) slots taken (low 32 bits) and
                                                    // overlap chunks (high 32 bits)
     int64_t total;                                 // K
-    int64_t sort_n;                                // min(K, key capacity)
     unsigned int big_tiles;                        // tiles sorted ahead of the raster (to 4096 keys)
     unsigned int huge_tiles;                       // those above 4096 keys
     int err;
     int overflow;                                  // the key or overlap list was too short: redo the frame
-    uint32_t epoch_scan, epoch_sort;               // look-back epochs of this frame
+    uint32_t epoch_scan;                           // look-back epoch of this frame
 };
 
 // The raster of at most so many tiles is launched while the sort before it
@@ -790,7 +789,6 @@ int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg
     ta.err = &dc->err;
     ta.total = &dc->total;
     ta.capacity = ctx->key_capacity;
-    ta.sort_n = &dc->sort_n;
     ta.overflow = &dc->overflow;
     ta.slot_counter = &dc->slots;
     ta.chunk_capacity = ctx->chunk_capacity;
@@ -1030,7 +1028,6 @@ int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, 
     for (;;) {
         ++attempts;
         ctx->h_init->epoch_scan = take_epochs(ctx->epoch_scan, 1, ctx->scan_status, st);
-        ctx->h_init->epoch_sort = 0;
         std::fill(ctx->h_result->t, ctx->h_result->t + kFrameTimes, 0ull);  // no older frame's time stands in
         // the second call with the same key is captured; a redone frame is not
         const bool use_graph = g && !g->failed && g->seen >= 2 && attempts == 1 && !ctx->tile_count_dirty;

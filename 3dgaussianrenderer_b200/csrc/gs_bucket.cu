@@ -48,31 +48,6 @@ __device__ __forceinline__ int64_t excl_scan_block(const int64_t v, int64_t* s_t
     return prefix + incl - v;
 }
 
-// OR and AND of one 64-bit value per thread over the block (pads pass
-// or_v = 0, and_v = ~0); every thread must call it.
-__device__ __forceinline__ uint64_t varying_bits_block(uint64_t or_v, uint64_t and_v, uint64_t* s_tmp)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-        or_v |= __shfl_xor_sync(kFull, or_v, o);
-        and_v &= __shfl_xor_sync(kFull, and_v, o);
-    }
-    if (lane == 0) {
-        s_tmp[warp] = or_v;
-        s_tmp[kWarps + warp] = and_v;
-    }
-    __syncthreads();
-    uint64_t o = 0, n = ~0ull;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-        o |= s_tmp[w];
-        n &= s_tmp[kWarps + w];
-    }
-    __syncthreads();
-    return o ^ n;
-}
-
 }  // namespace
 
 // Raster order: tiles go to the rasteriser by falling key count, in classes of
@@ -150,11 +125,8 @@ __global__ void __launch_bounds__(kThreads) tile_scan_kernel(const __grid_consta
         if (blk == nblk - 1) {
             const int64_t total = (int64_t)(prev + agg);
             *a.total = total;
-            if (a.sort_n) {
-                *a.sort_n = total < a.capacity ? total : a.capacity;
-                *a.overflow = total > a.capacity || (int64_t)(*a.slot_counter >> 32) > a.chunk_capacity ||
-                              (int64_t)*a.unit_count > a.unit_capacity;
-            }
+            *a.overflow = total > a.capacity || (int64_t)(*a.slot_counter >> 32) > a.chunk_capacity ||
+                          (int64_t)*a.unit_count > a.unit_capacity;
         }
     }
     __syncthreads();

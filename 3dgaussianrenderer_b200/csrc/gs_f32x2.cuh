@@ -25,12 +25,6 @@ __device__ __forceinline__ void f2_unpack(const f2 v, float& lo, float& hi)
 {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
-__device__ __forceinline__ f2 f2_add(const f2 a, const f2 b)
-{
-    f2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 __device__ __forceinline__ f2 f2_sub(const f2 a, const f2 b)
 {
     f2 d;

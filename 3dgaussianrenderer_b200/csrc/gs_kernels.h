@@ -242,7 +242,6 @@ struct TileScanArgs {
     int* err;
     int64_t* total;                  // K
     int64_t capacity;
-    int64_t* sort_n;                 // min(K, capacity)
     int* overflow;                   // K > capacity, or another list of the frame was too short
     const unsigned long long* slot_counter;
     int64_t chunk_capacity;
@@ -381,11 +380,8 @@ void launch_emit_bucket(const BucketEmitArgs& a, int num_sms, cudaStream_t st);
 void launch_tile_sort(const TileSortArgs& a, int num_sms, cudaStream_t st);
 void launch_large_overlaps(const FrameArgs& a, int num_sms, cudaStream_t st);
 void launch_count_stage(const FrameArgs& a, cudaStream_t st);
-// view_base[v] = sum of view_total[u < v]; *total = sum of all.  With a
-// non-null `sort_n`, also *sort_n = min(total, capacity) and *overflow = 1
-// when the keys do not fit (frames whose key count is not known on the host).
-void launch_view_base(const int64_t* view_total, int num_views, int64_t* view_base, int64_t* total, cudaStream_t st,
-                      int64_t capacity = 0, int64_t* sort_n = nullptr, int* overflow = nullptr);
+// view_base[v] = sum of view_total[u < v]; *total = sum of all.
+void launch_view_base(const int64_t* view_total, int num_views, int64_t* view_base, int64_t* total, cudaStream_t st);
 void launch_emit(const EmitArgs& a, cudaStream_t st);
 
 // Sorts num_items pairs on bits [0, key_bits).  When d_num_items is non-null

@@ -765,8 +765,7 @@ __global__ void __launch_bounds__(256) count_stage_kernel(FrameArgs a)
     }
 }
 
-__global__ void view_base_kernel(const int64_t* view_total, int num_views, int64_t* view_base, int64_t* total,
-                                 int64_t capacity, int64_t* sort_n, int* overflow)
+__global__ void view_base_kernel(const int64_t* view_total, int num_views, int64_t* view_base, int64_t* total)
 {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         int64_t run = 0;
@@ -775,10 +774,6 @@ __global__ void view_base_kernel(const int64_t* view_total, int num_views, int64
             run += view_total[v];
         }
         *total = run;
-        if (sort_n) {
-            *sort_n = run < capacity ? run : capacity;
-            *overflow = run > capacity ? 1 : 0;
-        }
     }
 }
 
@@ -968,10 +963,9 @@ void launch_count_stage(const FrameArgs& a, cudaStream_t st)
     count_stage_kernel<<<grid, 256, 0, st>>>(a);
 }
 
-void launch_view_base(const int64_t* view_total, int num_views, int64_t* view_base, int64_t* total, cudaStream_t st,
-                      int64_t capacity, int64_t* sort_n, int* overflow)
+void launch_view_base(const int64_t* view_total, int num_views, int64_t* view_base, int64_t* total, cudaStream_t st)
 {
-    view_base_kernel<<<1, 32, 0, st>>>(view_total, num_views, view_base, total, capacity, sort_n, overflow);
+    view_base_kernel<<<1, 32, 0, st>>>(view_total, num_views, view_base, total);
 }
 
 void launch_emit(const EmitArgs& a, cudaStream_t st)
