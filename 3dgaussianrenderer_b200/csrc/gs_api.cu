@@ -2,12 +2,13 @@
 // points (declared in include/gs_b200.h).
 //
 // Frame orchestration replaces the reference's frame loop
-// (app/main.cpp:326-432) and Renderer::Render (core/renderer.cpp:94-139):
-// everything runs on one stream with events between stages; the only host
-// synchronisation inside a frame is the read of the exact key count K after
-// the fused projection/count kernel (the reference syncs after every stage
-// and once more for its tile counter).  Buffers grow on demand and are
-// never truncated: the tile list is sized from the exact K.
+// (app/main.cpp:326-432) and Renderer::Render (core/renderer.cpp:94-139), which
+// sync after every stage and once more for the tile counter.  A bucket frame
+// (GS_ORDER_BUCKETS) is enqueued whole, or replayed as a graph, and the host
+// waits at its end; its kernels stamp the stage times.  A onesweep frame runs
+// on one stream with events between stages and one host read inside, of the
+// exact key count K after the fused projection/count kernel.  Buffers grow on
+// demand and are never truncated.
 #include "gs_kernels.h"
 #include "../../include/gs_b200.h"
 
@@ -716,9 +717,10 @@ int plan_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams,
 }
 
 // Enqueues a whole tile-bucket frame on `st` with no host synchronisation
-// (everything a replayed graph needs): counters reset, fused projection,
-// tile scan, bucket emit (which reports to ctx->h_result), tile sort, raster.  The key count stays on the device; a frame whose keys
-// exceed ctx->key_capacity comes back with `overflow` set.
+// (everything a replayed graph needs): counters reset, fused projection, large
+// splats, tile scan, bucket emit (which reports to ctx->h_result), tile sorts,
+// raster.  The key count stays on the device; a frame whose keys, overlap chunks
+// or large splats' units exceed their lists comes back with `overflow` set.
 int enqueue_bucket_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg& cfg, const FramePlan& p,
                          cudaStream_t st, bool capturing)
 {
@@ -967,7 +969,7 @@ bool capture_frame(gs_ctx* ctx, const gs_scene* scene, const gs_render_cfg& cfg,
 
 // One frame with GS_ORDER_BUCKETS.  The key count never goes to the host
 // before the frame ends: the lists are used at the capacity they have, and
-// a frame that outgrew them is redone once at 1.25x the count it reported.
+// a frame that outgrew them is redone at 1.25x the counts it reported.
 // With cfg.graph, the second frame with the same scene, options, view sizes
 // and outputs is captured into a CUDA graph and later ones replay it.
 int run_frame_bucket(gs_ctx* ctx, const gs_scene* scene, const gs_camera* cams, int num_views, const gs_render_cfg& cfg,

@@ -229,13 +229,14 @@ struct BucketEmitArgs {
     unsigned long long* batch_counter;  // chunks handed out; zero at launch
 };
 
-// Exclusive scan of the per-tile key counts into tile ranges; the last block writes the key total.  Ranges are clamped to
-// `capacity` (a frame whose keys do not fit is flagged, never overrun).
+// Exclusive scan of the per-tile key counts into tile ranges; the last block
+// writes the key total.  Ranges are clamped to `capacity` (a frame whose keys do
+// not fit is flagged, never overrun).
 struct TileScanArgs {
     uint32_t* count;                 // [tiles]; zeroed again after the scan
     int64_t tiles;
     int32_t* ranges;                 // [2 * tiles] out: first, one past last
-    uint64_t* status;                // look-back words, one per 4096 tiles
+    uint64_t* status;                // look-back words, one per kTileScanItems tiles
     unsigned long long* block_counter;
     uint32_t epoch;
     const uint32_t* epoch_dev;       // non-null: epoch read here
@@ -358,13 +359,13 @@ struct RasterArgs {
     const int32_t* slot_gi;
     int32_t fused_cap;
     const int32_t* order;             // the raster order of the tiles; null: as numbered
-    // record raster (GS_TERM_TMIN) knobs: entries between two tests of whether
-    // a block is done (32 or 64), and a persistent grid over the atomic tile queue
-    // (tile_counter, zero at launch) instead of one CTA per tile
     FrameResult* result;              // out: the raster's times; null: not wanted
     int32_t overlap;                  // 1: follows the sort directly, see launch_frame_step
     int32_t stamp_start;              // 1: the first CTA stamps the raster's start
     int32_t end_ctas;                 // the last so many CTAs stamp its end (and long tiles, stamp_end); 0: none
+    // record raster (GS_TERM_TMIN) knobs: entries between two tests of whether
+    // a block is done (32 or 64), and a persistent grid over the atomic tile queue
+    // (tile_counter, zero at launch) instead of one CTA per tile
     int32_t rec_chunk;
     int32_t rec_persistent;
     int32_t sort_prefix_bits;         // depth bits the fused tile sort radix-sorts (8..32; 0 = 16)

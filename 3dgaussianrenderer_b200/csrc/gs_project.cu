@@ -90,14 +90,7 @@ __device__ __forceinline__ unsigned lane_range_mask(const int lo, const int hi)
     return mhi & ~mlo;
 }
 
-// Returns this lane's number of overlapping tiles; for rectangles of at
-// most 32 candidates also the hit mask (bit c = candidate c overlaps).
-//
-// The overlap test is the reference's, in two phases: the walk decides every
-// candidate the cheap evaluation can call, and only if some candidate of the
-// warp was too close to call does a second walk settle those in IEEE
-// arithmetic.  Keeping the IEEE code out of the first walk keeps it free of
-// register spills.
+// Adds a step's ballot to this lane's hits and hit mask.
 __device__ __forceinline__ void add_hits(const unsigned bal, const WarpCands& w, const int base, const int cand,
                                          const int c0, int& hits, uint32_t& mask)
 {
@@ -157,6 +150,14 @@ __device__ __forceinline__ void owner_ell(const Ell& e, const int4 r, const int 
     orr.w = __shfl_sync(kFull, r.w, o);
 }
 
+// Returns this lane's number of overlapping tiles; for rectangles of at
+// most 32 candidates also the hit mask (bit c = candidate c overlaps).
+//
+// The overlap test is the reference's, in two phases: the walk decides every
+// candidate the cheap evaluation can call, and only if some candidate of the
+// warp was too close to call does a second walk settle those in IEEE
+// arithmetic, so that the first walk does not hold the IEEE code's registers
+// (one walk that calls it 6.81 against 6.25 ms on 64 views of 3M).
 __device__ __forceinline__ int warp_count_hits(const Ell& e, const int4 r, const int cand, const ViewParams& v,
                                                uint32_t& mask)
 {
@@ -520,7 +521,7 @@ __device__ __forceinline__ int64_t acquire_tile(unsigned long long* counter)
 //
 // BUCKET: no scan at all -- each (view, Gaussian) with candidate tiles takes a
 // slot and its overlaps go to the overlap list with their ranks in their
-// tiles (warp_bucket_hits); the blocks are independent and run in launch order.
+// tiles (start_walk, run_walk); the blocks are independent and run in launch order.
 __device__ __forceinline__ void sh_wait(uint64_t* bar, int* err)
 {
     int spins = 0;
@@ -575,8 +576,9 @@ __device__ __forceinline__ void write_record(float4* rec, const Ell& e, const fl
 // registers, and the copy is asked for only where a Gaussian is in view and
 // overlaps the walk (1080p view of 1M: 104 against 112 us; 64 views of 3M: 6.3
 // against 6.6 ms).
-// Blocks per SM: 4 (64 registers); the exact projection at SH degree 3
-// keeps 80 registers (3 blocks)
+// Blocks per SM: 4 (64 registers, at which the SH bucket forms spill 56 to 64
+// bytes a thread); the exact projection at SH degree 3 keeps 80 registers
+// (3 blocks)
 template <int DEG, bool BUCKET, bool FAST, bool MANY>
 __global__ void __launch_bounds__(256, (DEG >= 3 && !FAST) ? 3 : 4) frame_project_kernel(const __grid_constant__ FrameArgs a)
 {

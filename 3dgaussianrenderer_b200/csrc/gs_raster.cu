@@ -258,7 +258,7 @@ __device__ __forceinline__ const ViewParams& view_of_tile(const RasterArgs& a, c
 // packed f32x2 pair, so an entry's shared-memory reads (40 bytes, broadcast),
 // its row terms (dy, (c dy) dy) and its column terms (dx, a dx, 2 b dx) are
 // shared by the lane's pixels.
-// The FP32 pipe bounds the loop: 13 packed operations (two cycles each) and 6
+// The FP32 pipe bounds the loop (73 % busy on the frame below): 13 packed operations (two cycles each) and 6
 // scalar ones per entry and column pair.  On the 3M-Gaussian 1024x1024 frame
 // the raster takes 0.42 ms, against 0.55 ms with two pixels per lane in scalar
 // arithmetic (0.46 packed; 0.45 with four rows of one column per lane).
@@ -443,8 +443,9 @@ __device__ __forceinline__ int raster_ref_tile(const RasterArgs& a, const ViewPa
 }
 
 // One CTA per tile of every view, in the raster order when there is one.
-// 640 threads per SM (96 registers): the FP32 pipe is busy with 20 warps, and
-// more of them only slow the heaviest tiles down (768 threads: raster +3 %).
+// 640 threads per SM (96 registers, at which the wide lanes spill 76 bytes a
+// thread, 228 in 16x8 tiles): the FP32 pipe is busy with 20 warps, and more of
+// them only slow the heaviest tiles down (768 threads: raster +3 %).
 template <int TW, int TH, int COLS>
 __global__ void __launch_bounds__(RefShape<TW, TH, COLS>::NT, 640 / RefShape<TW, TH, COLS>::NT) raster_ref_kernel(RasterArgs a)
 {
@@ -507,12 +508,15 @@ __global__ void __launch_bounds__(TW * TH, 2048 / (TW * TH) * 5 / 8) raster_kern
 // and two pixels per lane those reads took 9 cycles of the SM's shared-memory
 // path per 64 evaluations and bound the loop; two blocks per warp, four
 // pixels per lane, halve them, share the row term (dy) and the column terms
-// (A dx^2 + L, B dx) among the pixels and leave the FP32 pipe (38 cycles per
-// entry of a warp, 63 % busy) and the ex2 unit (32 cycles, 53 %) as the bound.
+// (A dx^2 + L, B dx) among the pixels.  What is left is spread: on four views of
+// 3M Gaussians the issue slots are 67 % busy, the shared-memory path 66 %, the
+// FP32 pipe 63 % (38 cycles per entry of a warp) and the ex2 unit 53 % (32
+// cycles), and warps wait for one another's turn (not_selected, math_pipe_throttle).
 // Raster of the 64-view batch of 3M Gaussians 14.7 -> 12.8 ms, of eight
 // 1280x720 views of 1M 0.99 -> 0.83 ms, of one 1080p view 0.195 -> 0.175 ms.
-// 640 threads per SM (96 registers): 768 with 80 registers spill in the sort
-// and take 13.2 ms, 896 and 1024 take 14.0 ms.
+// 640 threads per SM (96 registers, at which the wide lanes spill 88 bytes a
+// thread, 132 in 16x8 tiles): 768 with 80 registers take 13.2 ms, 896 and 1024
+// take 14.0 ms.
 template <int TW, int TH, int BLOCKS>
 struct RecShape {
     static constexpr int BPW = BLOCKS;              // 8x8 blocks per warp, side by side
