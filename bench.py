@@ -34,9 +34,9 @@ VIEWS = 64
 N_GAUSS = 3_000_000
 # DRAM bytes (read + written) of the T_min raster launch of view 0 (1280x720)
 # rendered alone: ncu capture of the second frame of `bench.py --views 1
-# --steps 1 --warmup 1 --no-cpu --no-e2e --no-plain --no-serve` (128.2 MB
-# read, 7.0 MB written; the raster roofline's traffic)
-RASTER_VIEW0_TRAFFIC = 133.7e6
+# --steps 1 --warmup 1 --no-cpu --no-e2e --no-plain --no-serve` (120.4 MB
+# read, 5.2 MB written; the raster roofline's traffic)
+RASTER_VIEW0_TRAFFIC = 125.6e6
 RING_RADIUS = 15.0
 WORKLOAD = "3M Gaussians SH3, 64-view orbit ring r=15, 1280x720/1600x900/1920x1080 cycling, one batched frame"
 
@@ -566,13 +566,13 @@ def run_ours(args, rank, world, local_rank):
     # (32 B position + scale/rotation, 12 (d + 1)^2 = 192 B SH per Gaussian)
     # read once per block of `vpb` views, and the 48-byte splat record per
     # (view, Gaussian) of the scope table written: ceil(V / vpb) N 224 + V N 48.
-    # traffic: DRAM bytes of an ncu capture of a 4-view frame (684.2 MB read,
-    # 506.1 MB written), scaled to 64 views (reads per block of views, writes
-    # per view).  The kernel is issue-bound, far under this roof.
+    # traffic: DRAM bytes of an ncu capture of a 4-view frame (717.1 MB read,
+    # 574.1 MB written), scaled to 64 views (reads per block of views, writes
+    # per view).  The kernel is bound by latency and issue, far under this roof.
     vpb = min(VIEWS, rc.views_per_block or 16)
     blocks = (VIEWS + vpb - 1) // vpb
     alg_frame = blocks * N_GAUSS * (32 + 12 * 16) + VIEWS * N_GAUSS * 48
-    frame_traffic = 684.2e6 * blocks + 506.1e6 / 4 * VIEWS if VIEWS == 64 else None
+    frame_traffic = 717.1e6 * blocks + 574.1e6 / 4 * VIEWS if VIEWS == 64 else None
     frame_gbs = alg_frame / (per["project_ms"] / 1e3) / 1e9 if per["project_ms"] > 0 else None
     frame_roof = {"bound": "hbm", "kernel": "frame_project (SH + projection + tile counts)",
                   "achieved": frame_gbs, "peak": hbm, "unit": "GB/s",
